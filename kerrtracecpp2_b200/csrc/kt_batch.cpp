@@ -38,6 +38,7 @@ struct Group {
   kt::Mode fb_mode = kt::kModeBLRk4;  // BL launch over the fallback list
   std::vector<int> frames;  // batch frame indices
   bool fp32 = false;        // some frame may run the mixed FP32 right-hand side
+  bool lam = false;         // some frame has Lambda != 0
   uint64_t n_rays = 0;
   kt::Frame* d_frames = nullptr;
   kt::OutSoA* d_outs = nullptr;
@@ -97,6 +98,7 @@ kt::BatchRays group_rays(const Group& g, const uint32_t* list, const uint32_t* n
   br.n_dev = n_dev;
   br.n = n;
   br.fp32 = g.fp32;
+  br.lam = g.lam;
   return br;
 }
 
@@ -315,6 +317,7 @@ kt_status kt_batch_create(kt_context* ctx, const kt_frame_desc* descs, const kt_
     Group& g = b->groups[group_of_key[key]];
     g.frames.push_back(i);
     g.fp32 = g.fp32 || std::isfinite(frames[i].r_fp32);
+    g.lam = g.lam || frames[i].g.L != 0.0;
     if (frames[i].solver == KT_SOLVER_ELLIPTIC_CLOSED) {
       g.ell_frames.push_back(frames[i]);
       g.ell_outs.push_back(to_out(&outs[i]));

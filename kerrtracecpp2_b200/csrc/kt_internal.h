@@ -139,6 +139,9 @@ struct BatchRays {
   // some frame may run the mixed tracer's FP32 right-hand side (a finite
   // r_fp32): selects the mixed kernels that carry the FP32 branch
   bool fp32 = true;
+  // some frame has Lambda != 0: selects the exact BL kernels that carry
+  // Delta_theta and Xi (without it both are 1)
+  bool lam = true;
 };
 
 // Launch-shape variants the batch autotuner chooses from: (threads per

@@ -7,10 +7,14 @@
 
 namespace kt {
 
-struct ModeBLRk4 {
-  using Machine = BLRk4;
-  static constexpr int kSlots = BLRk4::kSlots;
-  BLRk4* m;
+// The BL modes come in two instantiations: kLam = false for launches whose
+// frames all have Lambda = 0 (bl_rhs_exact; 640 x 360 DOPRI5 without Lambda:
+// 14.6 ms, and 14.7 to 15.9 with the Lambda kernel).
+template <class M, bool kLam>
+struct ModeBL {
+  using Machine = M;
+  static constexpr int kSlots = M::kSlots;
+  M* m;
   __device__ __forceinline__ bool needs_k1() const { return m->needs_k1(); }
   __device__ __forceinline__ bool start(const Frame& f, uint32_t pix, uint32_t, uint32_t, const Fallback&) {
     m->init(f, camera_ray(f, pix));
@@ -19,27 +23,13 @@ struct ModeBLRk4 {
   __device__ __forceinline__ bool slot(const Frame& f, int s, RayResult* res) {
     double y[4], k[5];
     m->input(s, y);
-    bl_rhs(f.g, y[0], y[1], y[2], y[3], m->pt, m->pphi, k);
+    if (!bl_rhs_exact<kLam>(f.g, y[0], y[1], y[2], y[3], m->pt, m->pphi, k))
+      bl_rhs_rest(f.g, y[0], y[1], y[2], y[3], m->pt, m->pphi, k);
     return m->consume(f, s, k, res);
   }
 };
-
-struct ModeBLDopri5 {
-  using Machine = BLDopri5;
-  static constexpr int kSlots = BLDopri5::kSlots;
-  BLDopri5* m;
-  __device__ __forceinline__ bool needs_k1() const { return m->needs_k1(); }
-  __device__ __forceinline__ bool start(const Frame& f, uint32_t pix, uint32_t, uint32_t, const Fallback&) {
-    m->init(f, camera_ray(f, pix));
-    return true;
-  }
-  __device__ __forceinline__ bool slot(const Frame& f, int s, RayResult* res) {
-    double y[4], k[5];
-    m->input(s, y);
-    bl_rhs(f.g, y[0], y[1], y[2], y[3], m->pt, m->pphi, k);
-    return m->consume(f, s, k, res);
-  }
-};
+template <bool kLam> using ModeBLRk4 = ModeBL<BLRk4, kLam>;
+template <bool kLam> using ModeBLDopri5 = ModeBL<BLDopri5, kLam>;
 
 struct ModeKSRk4 {
   using Machine = KSRk4;
@@ -158,27 +148,20 @@ struct ModeSepRk4 {
 template <> struct Defers<ModeSepRk4> { static constexpr bool value = true; };
 
 // Launch shape per mode, measured on B200 (720p config-2 frame, BL chart
-// DOPRI5 and RK4; 720p Kerr KS frame; 1080p config-3 bundles): the BL and KS
-// single-ray kernels run best as 64-thread blocks capped at 113 registers
+// DOPRI5 and RK4; 720p Kerr KS frame; 1080p config-3 bundles): the KS
+// kernel runs best as 64-thread blocks capped at 113 registers
 // (9 blocks per SM), the bundle kernel as 128-thread blocks.  Refilling a
 // warp only once all its lanes are idle (kRefill 32) keeps the 32 rays of a
 // warp neighbouring pixels that start together: the camera set-up and the
 // first slots run converged and the rays' step sequences stay alike, which
 // outweighs the lanes idling at the end of each group of 32 (KS: 62 against
 // 73 ms, BL RK4: 66 against 68, DOPRI5: equal; bundles best at 16).
-template <> struct Shape<struct ModeBLRk4> { static constexpr int kBlock = 64, kMinBlocks = 9, kRefill = 32; };
-#ifndef KT_BL_DOPRI5_MINB
-#define KT_BL_DOPRI5_MINB 9
-#endif
-#ifndef KT_BL_DOPRI5_REFILL
-#define KT_BL_DOPRI5_REFILL 32
-#endif
-#ifndef KT_BL_DOPRI5_BLOCK
-#define KT_BL_DOPRI5_BLOCK 64
-#endif
-template <> struct Shape<struct ModeBLDopri5> {
-  static constexpr int kBlock = KT_BL_DOPRI5_BLOCK, kMinBlocks = KT_BL_DOPRI5_MINB,
-                       kRefill = KT_BL_DOPRI5_REFILL;
+// The BL kernels with bl_rhs_exact: 8 blocks (16 warps) per SM at 128
+// registers without a spill.  720p DOPRI5 41.1 ms against 43.0 with 10 blocks
+// (96 registers, 22 B spilled) and 43.4 with 6; RK4 at 641 x 359 9.4 / 10.7 /
+// 8.8 ms (that frame is short enough for its longest rays to show).
+template <class M, bool kLam> struct Shape<ModeBL<M, kLam>> {
+  static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32;
 };
 template <> struct Shape<struct ModeKSRk4> { static constexpr int kBlock = 64, kMinBlocks = 9, kRefill = 32; };
 template <> struct Shape<struct ModeBundle> { static constexpr int kBlock = 128, kMinBlocks = 1, kRefill = 16; };
@@ -197,11 +180,19 @@ template <> struct Shape<ModeBundlePair> {
                        kRefill = KT_BUNDLE_PAIR_REFILL;
 };
 
+template <class ModeT>
+static cudaError_t launch_one(const Frame& f, const OutSoA& out, const RayList& rl,
+                              uint32_t* queue, const Fallback& fb, const LaunchShape& s,
+                              cudaStream_t stream) {
+  k_trace<ModeT><<<s.grid, s.block, s.smem, stream>>>(f, out, rl, queue, fb);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_shape(Mode mode, int device, LaunchShape* shape) {
   if (is_mixed_mode(mode)) return launch_shape_mixed(mode, device, shape);
   switch (mode) {
-    case kModeBLRk4: return shape_for<ModeBLRk4>(device, shape);
-    case kModeBLDopri5: return shape_for<ModeBLDopri5>(device, shape);
+    case kModeBLRk4: return shape_for_both<ModeBLRk4<true>, ModeBLRk4<false>>(device, shape);
+    case kModeBLDopri5: return shape_for_both<ModeBLDopri5<true>, ModeBLDopri5<false>>(device, shape);
     case kModeKSRk4: return shape_for<ModeKSRk4>(device, shape);
     case kModeBundle: return shape_for_pair<ModeBundlePair>(device, shape);
     case kModeSepRk4: return shape_for<ModeSepRk4>(device, shape);
@@ -213,12 +204,17 @@ cudaError_t launch_trace(Mode mode, const Frame& f, const OutSoA& out, const Ray
                          uint32_t* queue, const Fallback& fb, const LaunchShape& s,
                          cudaStream_t stream) {
   if (is_mixed_mode(mode)) return launch_trace_mixed(mode, f, out, rl, queue, fb, s, stream);
+  const bool lam = f.g.L != 0.0;
   switch (mode) {
-    case kModeBLRk4: k_trace<ModeBLRk4><<<s.grid, s.block, s.smem, stream>>>(f, out, rl, queue, fb); break;
-    case kModeBLDopri5: k_trace<ModeBLDopri5><<<s.grid, s.block, s.smem, stream>>>(f, out, rl, queue, fb); break;
-    case kModeKSRk4: k_trace<ModeKSRk4><<<s.grid, s.block, s.smem, stream>>>(f, out, rl, queue, fb); break;
+    case kModeBLRk4:
+      return lam ? launch_one<ModeBLRk4<true>>(f, out, rl, queue, fb, s, stream)
+                 : launch_one<ModeBLRk4<false>>(f, out, rl, queue, fb, s, stream);
+    case kModeBLDopri5:
+      return lam ? launch_one<ModeBLDopri5<true>>(f, out, rl, queue, fb, s, stream)
+                 : launch_one<ModeBLDopri5<false>>(f, out, rl, queue, fb, s, stream);
+    case kModeKSRk4: return launch_one<ModeKSRk4>(f, out, rl, queue, fb, s, stream);
     case kModeBundle: k_trace_pair<ModeBundlePair><<<s.grid, s.block, s.smem, stream>>>(f, out, rl, queue, fb); break;
-    case kModeSepRk4: k_trace<ModeSepRk4><<<s.grid, s.block, s.smem, stream>>>(f, out, rl, queue, fb); break;
+    case kModeSepRk4: return launch_one<ModeSepRk4>(f, out, rl, queue, fb, s, stream);
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -226,8 +222,9 @@ cudaError_t launch_trace(Mode mode, const Frame& f, const OutSoA& out, const Ray
 
 cudaError_t batch_shape(Mode mode, int variant, int device, LaunchShape* shape) {
   switch (mode) {
-    case kModeBLRk4: return batch_shape<ModeBLRk4>(variant, device, shape);
-    case kModeBLDopri5: return batch_shape<ModeBLDopri5>(variant, device, shape);
+    case kModeBLRk4: return batch_shape_both<ModeBLRk4<true>, ModeBLRk4<false>>(variant, device, shape);
+    case kModeBLDopri5:
+      return batch_shape_both<ModeBLDopri5<true>, ModeBLDopri5<false>>(variant, device, shape);
     case kModeKSRk4: return batch_shape<ModeKSRk4>(variant, device, shape);
     case kModeBundle:
       if (variant == kBatchPairVariant)
@@ -242,8 +239,12 @@ cudaError_t batch_shape(Mode mode, int variant, int device, LaunchShape* shape) 
 cudaError_t launch_batch(Mode mode, int variant, const BatchRays& br, uint32_t* queue,
                          const Fallback& fb, const LaunchShape& s, cudaStream_t st) {
   switch (mode) {
-    case kModeBLRk4: return batch_launch<ModeBLRk4>(variant, br, queue, fb, s, st);
-    case kModeBLDopri5: return batch_launch<ModeBLDopri5>(variant, br, queue, fb, s, st);
+    case kModeBLRk4:
+      return br.lam ? batch_launch<ModeBLRk4<true>>(variant, br, queue, fb, s, st)
+                    : batch_launch<ModeBLRk4<false>>(variant, br, queue, fb, s, st);
+    case kModeBLDopri5:
+      return br.lam ? batch_launch<ModeBLDopri5<true>>(variant, br, queue, fb, s, st)
+                    : batch_launch<ModeBLDopri5<false>>(variant, br, queue, fb, s, st);
     case kModeKSRk4: return batch_launch<ModeKSRk4>(variant, br, queue, fb, s, st);
     case kModeBundle:
       if (variant == kBatchPairVariant) {

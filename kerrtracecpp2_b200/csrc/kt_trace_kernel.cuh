@@ -240,6 +240,18 @@ static cudaError_t shape_for(int device, LaunchShape* shape) {
   return cudaSuccess;
 }
 
+// One shape for two instantiations of a mode with the same launch bounds and
+// record (a launch takes either): the larger grid, whose surplus blocks find
+// the queue empty.
+template <class A, class B>
+static cudaError_t shape_for_both(int device, LaunchShape* shape) {
+  LaunchShape b;
+  cudaError_t e = shape_for<A>(device, shape);
+  if (e == cudaSuccess) e = shape_for<B>(device, &b);
+  if (e == cudaSuccess && b.grid > shape->grid) shape->grid = b.grid;
+  return e;
+}
+
 // ---- batches of frames -----------------------------------------------------
 // Many frames (parameter sets, resolutions) in one persistent launch
 // (BatchRays, kt_internal.h).  Each lane carries its own frame index; the
@@ -423,6 +435,16 @@ static cudaError_t batch_shape(int variant, int device, LaunchShape* s) {
     case 2: return batch_shape_for<ModeT, 64, 12>(device, s);
   }
   return cudaErrorInvalidValue;
+}
+
+// As shape_for_both.
+template <class A, class B>
+static cudaError_t batch_shape_both(int variant, int device, LaunchShape* s) {
+  LaunchShape b;
+  cudaError_t e = batch_shape<A>(variant, device, s);
+  if (e == cudaSuccess) e = batch_shape<B>(variant, device, &b);
+  if (e == cudaSuccess && b.grid > s->grid) s->grid = b.grid;
+  return e;
 }
 
 template <class ModeT>

@@ -93,8 +93,18 @@ KTM_FN double ktm_scale(double x, int n) {
 
 /* Reduced-argument kernels for r = rh + rl, |rh| <= pi/4 (+ a few ulp),
  * |rl| <= ulp(rh): sin(rh+rl) ~ sin(rh) + rl cos(rh), cos ~ cos(rh) - rl sin(rh). */
+/* On the device the coefficients sit in constant memory: as literals each
+ * one costs two moves into uniform registers per use. */
+#if defined(__CUDACC__)
+static __constant__ double ktm_sin_c[9] = KTM_SIN_COEFFS;
+static __constant__ double ktm_cos_c[9] = KTM_COS_COEFFS;
+#endif
 KTM_FN double ktm_sin_kernel(double rh, double rl) {
+#if defined(__CUDA_ARCH__)
+  const double* c = ktm_sin_c;
+#else
   const double c[9] = KTM_SIN_COEFFS;
+#endif
   const double z = rh * rh;
   double p = c[8];
   p = fma(p, z, c[7]);
@@ -109,7 +119,11 @@ KTM_FN double ktm_sin_kernel(double rh, double rl) {
 }
 
 KTM_FN double ktm_cos_kernel(double rh, double rl) {
+#if defined(__CUDA_ARCH__)
+  const double* c = ktm_cos_c;
+#else
   const double c[9] = KTM_COS_COEFFS;
+#endif
   const double z = rh * rh;
   const double zlo = fma(rh, rh, -z);
   double p = c[8];
@@ -159,7 +173,43 @@ KTM_FN void ktm_rem_pio2(double x, double* rh, double* rl, int* q) {
   *q = (int)((int64_t)k & 3);
 }
 
-KTM_FN void ktm_sincos(double x, double* s, double* c) {
+/* sin and cos for 2^-27 <= |x| < 2^26, where ktm_rem_pio2 needs no case
+ * distinctions: the quadrant count k = rint(x 2/pi) by adding and subtracting
+ * 1.5 2^52 (the same integer, and its low bits are the sum's low word), and
+ * no separate path below pi/4, where k = 0 makes the reduction return x
+ * itself and a zero tail.  Bit for bit ktm_sincos_any; on the device this
+ * saves the double-to-integer conversion, the range comparisons in the FP64
+ * pipe and two divergent branches. */
+#if defined(__CUDA_ARCH__)
+#define KTM_MUL_RN(a, b) __dmul_rn(a, b)
+#define KTM_ADD_RN(a, b) __dadd_rn(a, b)
+#else
+#define KTM_MUL_RN(a, b) ((a) * (b))
+#define KTM_ADD_RN(a, b) ((a) + (b))
+#endif
+KTM_FN int ktm_sincos_plain(double x) {
+  return ((uint32_t)(ktm_bits(x) >> 32) & 0x7fffffffu) - 0x3e400000u < 0x41900000u - 0x3e400000u;
+}
+KTM_FN void ktm_sincos_core(double x, double* s, double* c) {
+  const double kMagic = 0x1.8p52;
+  const double t0 = KTM_ADD_RN(KTM_MUL_RN(x, KTM_2_OVER_PI), kMagic);
+  const double k = KTM_ADD_RN(t0, -kMagic);
+  const uint32_t q = (uint32_t)ktm_bits(t0);
+  const double r1 = fma(-k, KTM_PIO2_1, x);
+  const double t = k * KTM_PIO2_2;
+  const double tl = fma(k, KTM_PIO2_2, -t);
+  const double h = r1 - t;
+  const double l = (((r1 - h) - t) - tl) - k * KTM_PIO2_3;
+  const double rh = h + l;
+  const double rl = (h - rh) + l;
+  const double sr = ktm_sin_kernel(rh, rl);
+  const double cr = ktm_cos_kernel(rh, rl);
+  const double a = (q & 1u) ? cr : sr, b = (q & 1u) ? sr : cr;
+  *s = ktm_from_bits(ktm_bits(a) ^ ((uint64_t)(q & 2u) << 62));
+  *c = ktm_from_bits(ktm_bits(b) ^ ((uint64_t)((q + 1u) & 2u) << 62));
+}
+
+KTM_FN void ktm_sincos_any(double x, double* s, double* c) {
   if (fabs(x) < 0x1p-27) {
     *s = x;
     *c = 1.0;
@@ -176,6 +226,19 @@ KTM_FN void ktm_sincos(double x, double* s, double* c) {
     case 2: *s = -sr; *c = -cr; break;
     default: *s = -cr; *c = sr; break;
   }
+}
+
+/* The other arguments (tiny, huge, Inf, NaN) are a real call on the device. */
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__ void ktm_sincos_rest(double x, double* s, double* c) {
+  ktm_sincos_any(x, s, c);
+}
+#else
+#define ktm_sincos_rest ktm_sincos_any
+#endif
+KTM_FN void ktm_sincos(double x, double* s, double* c) {
+  if (ktm_sincos_plain(x)) ktm_sincos_core(x, s, c);
+  else ktm_sincos_rest(x, s, c);
 }
 
 KTM_FN double ktm_sin(double x) {

@@ -1,0 +1,65 @@
+// kt_exactcheck.cpp -- TEST-ONLY host build of the exact right-hand sides'
+// fast forms (kt_exact.cuh, bl_rhs_exact, ktm_sincos_core), compared bit for
+// bit with the general forms.  Built by test_exact.py with -ffp-contract=off.
+#include <string.h>
+
+#include "../kerrtracecpp2_b200/csrc/kt_machines.cuh"
+
+using namespace kt;
+
+extern "C" {
+
+// Quotients a[i]/b[i] by kt_exact.cuh against the division; returns the
+// number that differ, and how many denominators its range test refuses.
+long ec_quot(long n, const double* a, const double* b, long* refused) {
+  long bad = 0;
+  *refused = 0;
+  for (long i = 0; i < n; ++i) {
+    if (top_ones(b[i]) & kTopBit) {
+      ++*refused;
+      continue;
+    }
+    const Rcp R = make_rcp(b[i]);
+    const double q = quot_signed(a[i], R), e = a[i] / b[i];
+    if (memcmp(&q, &e, 8) != 0) ++bad;
+    const double q1 = quot_one(R), e1 = 1.0 / b[i];
+    if (memcmp(&q1, &e1, 8) != 0) ++bad;
+  }
+  return bad;
+}
+
+long ec_sincos(long n, const double* x, long* plain) {
+  long bad = 0;
+  *plain = 0;
+  for (long i = 0; i < n; ++i) {
+    double s, c, s2, c2;
+    ktm_sincos(x[i], &s, &c);
+    ktm_sincos_any(x[i], &s2, &c2);
+    *plain += ktm_sincos_plain(x[i]);
+    if (memcmp(&s, &s2, 8) != 0 || memcmp(&c, &c2, 8) != 0) ++bad;
+  }
+  return bad;
+}
+
+// States y[i] = (r, theta, p_r, p_theta, p_t, p_phi) in one metric: how many
+// bl_rhs_exact results differ from bl_rhs; *refused counts those it hands back.
+long ec_bl_rhs(double M, double a, double Q, double L, int lam, long n, const double* y,
+               long* refused) {
+  const Metric g = make_metric(M, a, Q, L);
+  long bad = 0;
+  *refused = 0;
+  for (long i = 0; i < n; ++i) {
+    const double* s = y + 6 * i;
+    double k[5], e[5];
+    const bool ok = lam ? bl_rhs_exact<true>(g, s[0], s[1], s[2], s[3], s[4], s[5], k)
+                        : bl_rhs_exact<false>(g, s[0], s[1], s[2], s[3], s[4], s[5], k);
+    if (!ok) {
+      ++*refused;
+      continue;
+    }
+    bl_rhs(g, s[0], s[1], s[2], s[3], s[4], s[5], e);
+    if (memcmp(k, e, sizeof k) != 0) ++bad;
+  }
+  return bad;
+}
+}
