@@ -99,7 +99,7 @@ def copy_reference(reference):
 
 
 def build_reference(reference, force=False):
-    if not os.path.isdir(reference):
+    if not os.path.exists(os.path.join(reference, REF_FILES[0])):
         print(f"reference tree {reference} absent: using prebuilt oracle/_ref if present")
         return None
     src_dir = copy_reference(reference)
@@ -139,7 +139,7 @@ def build_reference_main_cuda(reference, force=False):
     output goes to the working directory (OUT_DIR ".")."""
     lib_dir = os.path.join(ROOT, "kerrtracecpp2_b200")
     lib = os.path.join(lib_dir, "libkerrtrace.so")
-    if not os.path.isdir(reference) or not os.path.exists(lib):
+    if not os.path.exists(os.path.join(reference, REF_FILES[0])) or not os.path.exists(lib):
         return None
     src_dir = copy_reference(reference)
     inc = os.path.join(REF_OUT, "cuda_inc", "gpu", "cuda")
