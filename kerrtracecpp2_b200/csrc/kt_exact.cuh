@@ -26,7 +26,8 @@
 // q0 = RN(a y2), which can be 1.5 ulp off, the bound fails for b_m > 1.15.)
 // The excluded significands (the top 18 bits all ones) are part of the
 // range test; their quotients take the division.  Nothing over- or
-// underflows for |b| and non-zero |a| in [2^-450, 2^450].
+// underflows for |b| in [2^-300, 2^300] and non-zero |a| in [2^-500, 2^500]
+// (the smallest intermediate, a residual, is 2^-106 |a|).
 #pragma once
 
 #include "ktmath.h"
@@ -59,7 +60,7 @@ KT_EX bool in_range(double x, int k) {
   const uint32_t lo = (uint32_t)(1023 - k) << 20, span = (uint32_t)(2 * k) << 20;
   return (hi_word(x) & 0x7fffffffu) - lo < span;
 }
-KT_EX bool is_zero(double x) { return ((hi_word(x) << 1) | lo_word(x)) == 0u; }
+KT_EX bool is_zero(double x) { return ((hi_word(x) & 0x7fffffffu) | lo_word(x)) == 0u; }
 
 // Bit kTopBit is set when the significand's top 18 bits are all ones.
 constexpr uint32_t kTopBit = 1u << 20;
@@ -101,5 +102,66 @@ KT_EX double quot(double a, const Rcp& R) {
 KT_EX double quot_signed(double a, const Rcp& R) { return is_zero(a) ? a * R.y1 : quot(a, R); }
 // RN(1 / b): q1 is y2.
 KT_EX double quot_one(const Rcp& R) { return fma(fma(-R.b, R.y2, 1.0), R.y2, R.y2); }
+
+// A denominator whose reciprocal is known within 2^-38 already.
+KT_EX Rcp make_rcp_from(double b, double y1) {
+  Rcp R;
+  R.b = b;
+  R.y1 = y1;
+  R.y2 = fma(fma(-b, y1, 1.0), y1, y1);
+  return R;
+}
+
+// ---- square roots ----------------------------------------------------------
+// RN(sqrt(x)), and 1/sqrt(x) within 2^-52, which the quotients by the root
+// and by its square start from (make_rcp_from).  Markstein's correction
+// g + (x - g^2) h of an approximate root g, h = 1/(2 sqrt(x)):
+//   y0 = 1/sqrt(x) within 2^-19 (the hardware seed); e = 1 - x y0^2, whose
+//   rounding of x y0 leaves an error of 2^-53; y = y0 (1 + e/2 + 3 e^2/8),
+//   within 1.6 x 2^-53 of 1/sqrt(x) (series 2^-58, e 2^-54, rounding 2^-53);
+//   g = RN(x y), then two corrections with h = y/2.
+// The first leaves g within (1/2 + 2^-40) ulp.  For the second write, with
+// u = ulp(g) and x scaled into [1, 4), g = K u and x - g^2 = D u^2 (exact in
+// the fma): sqrt(x) < g + u/2 means D <= K, and the result stays at g when
+// |D| (1 + d) < K, d = 2 g h - 1, |d| <= 1.6 x 2^-53.  x is a multiple of
+// 2^52 u^2, so K^2 + D is one of 2^52; with D = +-(K - j) or +-(K + j) that
+// makes j even, and j = 0 only for K = 2^52 and K = 2^53 - 1, that is x next
+// to a power of four, which the range test hands to sqrt().  From j >= 2
+// on, |D| and K differ by 2/K >= 2^-52 > |d|, so the comparison is decided
+// as the exact root decides it.
+KT_EX double rsqrt_seed(double x) {
+#if defined(__CUDA_ARCH__)
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+#else
+  return ktm_from_bits(ktm_bits(1.0 / sqrt(x)) & 0xffffffff00000000ull);
+#endif
+}
+struct Root {
+  double g, y;  // RN(sqrt(x)); 1/sqrt(x) within 2^-52
+};
+KT_EX Root make_root(double x) {
+  Root R;
+  const double y0 = rsqrt_seed(x);
+  const double e = fma(-(x * y0), y0, 1.0);
+  R.y = fma(y0 * e, fma(0.375, e, 0.5), y0);
+  const double h = 0.5 * R.y;
+  double g = x * R.y;
+  g = fma(fma(-g, g, x), h, g);
+  R.g = fma(fma(-g, g, x), h, g);
+  return R;
+}
+// Bit kTopBit is set when the significand's top 18 bits are all ones or all
+// zeros.
+KT_EX uint32_t top_edge(double x) {
+  const uint32_t h = hi_word(x);
+  return ((h + 4u) ^ h) | ((h - 4u) ^ h);
+}
+// 2^-k <= x < 2^k (positive).
+KT_EX bool in_range_pos(double x, int k) {
+  const uint32_t lo = (uint32_t)(1023 - k) << 20, span = (uint32_t)(2 * k) << 20;
+  return hi_word(x) - lo < span;
+}
 
 }  // namespace kt

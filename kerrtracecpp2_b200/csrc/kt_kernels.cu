@@ -49,7 +49,8 @@ struct ModeKSRk4 {
   __device__ __forceinline__ bool slot(const Frame& f, int s, RayResult* res) {
     double y[6], k[6];
     m->input(s, y);
-    ks_rhs(f.g, y[0], y[1], y[2], y[3], y[4], y[5], m->pT, k);
+    if (!ks_rhs_exact(f.g, y[0], y[1], y[2], y[3], y[4], y[5], m->pT, k))
+      ks_rhs_rest(f.g, y[0], y[1], y[2], y[3], y[4], y[5], m->pT, k);
     return m->consume(f, s, k, res);
   }
 };
@@ -148,14 +149,15 @@ struct ModeSepRk4 {
 template <> struct Defers<ModeSepRk4> { static constexpr bool value = true; };
 
 // Launch shape per mode, measured on B200 (720p config-2 frame, BL chart
-// DOPRI5 and RK4; 720p Kerr KS frame; 1080p config-3 bundles): the KS
-// kernel runs best as 64-thread blocks capped at 113 registers
-// (9 blocks per SM), the bundle kernel as 128-thread blocks.  Refilling a
+// DOPRI5 and RK4; 720p Kerr KS frame; 1080p config-3 bundles): the BL and KS
+// single-ray kernels run best as 64-thread blocks, 8 per SM, the bundle
+// kernel as 128-thread blocks.  Refilling a
 // warp only once all its lanes are idle (kRefill 32) keeps the 32 rays of a
 // warp neighbouring pixels that start together: the camera set-up and the
 // first slots run converged and the rays' step sequences stay alike, which
-// outweighs the lanes idling at the end of each group of 32 (KS: 62 against
-// 73 ms, BL RK4: 66 against 68, DOPRI5: equal; bundles best at 16).
+// outweighs the lanes idling at the end of each group of 32 (with the
+// division-based right-hand sides, KS: 62 against 73 ms, BL RK4: 66 against
+// 68, DOPRI5: equal; bundles best at 16).
 // The BL kernels with bl_rhs_exact: 8 blocks (16 warps) per SM at 128
 // registers without a spill.  720p DOPRI5 41.1 ms against 43.0 with 10 blocks
 // (96 registers, 22 B spilled) and 43.4 with 6; RK4 at 641 x 359 9.4 / 10.7 /
@@ -163,7 +165,8 @@ template <> struct Defers<ModeSepRk4> { static constexpr bool value = true; };
 template <class M, bool kLam> struct Shape<ModeBL<M, kLam>> {
   static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32;
 };
-template <> struct Shape<struct ModeKSRk4> { static constexpr int kBlock = 64, kMinBlocks = 9, kRefill = 32; };
+// (720p KS frame 51.6 ms against 52.3 with 10 blocks of 96 registers.)
+template <> struct Shape<struct ModeKSRk4> { static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32; };
 template <> struct Shape<struct ModeBundle> { static constexpr int kBlock = 128, kMinBlocks = 1, kRefill = 16; };
 // Paired bundles: 64 rays per 128-thread block; kRefill counts lanes.
 #ifndef KT_BUNDLE_PAIR_BLOCK

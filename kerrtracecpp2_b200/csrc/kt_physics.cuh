@@ -393,7 +393,7 @@ KT_HD bool bl_rhs_exact(const Metric& g, double r, double th, double pr, double 
   const double eps_r = 1e-5 * dmax(fabs(r), 0.01);
   const double eps_th = 1e-6;
   uint32_t top = 0;
-  bool ok = (g.tame != 0) & ((hi_word(r) >> 31) == 0) & in_range(r, 40);
+  bool ok = (g.tame != 0) & in_range_pos(r, 40);
   const double pt2 = 2.0 * pt;
   const BLAng A0 = bl_ang_exact<kLam>(g, th);
   const BLRad R0 = bl_rad<kLam>(g, r);
@@ -966,6 +966,118 @@ KT_HD void ks_rhs(const Metric& g, double X, double Y, double Z, double pX, doub
   k[3] = -(h1 - h2) / (2.0 * eX);
   k[4] = -(h3 - h4) / (2.0 * eY);
   k[5] = -(h5 - h6) / (2.0 * eZ);
+}
+
+// ks_rhs as the exact kernels evaluate it: the same arithmetic, bit for bit,
+// with the square roots and quotients of kt_exact.cuh and without the
+// products that are trivial.  l^0 = -1, so g^{0i} = g^{i0} = H l^i and g^00 =
+// -1 - H; the zeros of eta only turn signs, which the products carry.  The
+// 1/2 of H moves into the divisor 4 eps.
+//
+// One point of the finite-difference stencil: H's factors at (X, Y, Z).
+// kCentre keeps the division's sign of a zero (only in dX/dlambda can it
+// reach a result; H never cancels to a signed zero).
+struct KSPoint {
+  double H, l1, l2, l3;
+};
+template <bool kCentre>
+KT_HD KSPoint ks_point(const Metric& g, double X, double Y, double Z, uint32_t* top, bool* ok) {
+  const double R2 = (X * X + Y * Y) + Z * Z;
+  const double b = R2 - g.a2;
+  const double x1 = b * b + (g.fa2 * Z) * Z;
+  const Root r1 = make_root(x1);
+  const double x2 = 0.5 * (b + r1.g);
+  const Root r2 = make_root(x2);
+  const double r = r2.g;
+  const double r_sq = r * r;
+  const Rcp Rr = make_rcp_from(r, r2.y), Rs = make_rcp_from(r_sq, r2.y * r2.y);
+  const double rho2 = r_sq + quot((g.a2 * Z) * Z, Rs);
+  const double r2a2 = r_sq + g.a2;
+  const Rcp Ro = make_rcp(rho2), Ra = make_rcp(r2a2);
+  KSPoint P;
+  P.H = quot(g.twoM * r - g.Q2, Ro);
+  const double n1 = r * X + g.a * Y, n2 = r * Y - g.a * X;
+  P.l1 = kCentre ? quot_signed(n1, Ra) : quot(n1, Ra);
+  P.l2 = kCentre ? quot_signed(n2, Ra) : quot(n2, Ra);
+  P.l3 = kCentre ? quot_signed(Z, Rr) : quot(Z, Rr);
+  *top |= top_edge(x1) | top_edge(x2) | top_ones(r) | top_ones(r_sq) | top_ones(rho2) | top_ones(r2a2);
+  *ok = *ok & in_range_pos(x1, 300) & in_range_pos(x2, 80);
+  return P;
+}
+
+// 2 H_ham at a point, summed in ks_ham's order.
+KT_HD double ks_ham2(const KSPoint& P, double pT, double pX, double pY, double pZ) {
+  const double h1 = P.H * P.l1, h2 = P.H * P.l2, h3 = P.H * P.l3;
+  double H = ((-1.0 - P.H) * pT) * pT;
+  H += (h1 * pT) * pX;
+  H += (h2 * pT) * pY;
+  H += (h3 * pT) * pZ;
+  H += (h1 * pX) * pT;
+  H += ((1.0 - h1 * P.l1) * pX) * pX;
+  H -= ((h1 * P.l2) * pX) * pY;
+  H -= ((h1 * P.l3) * pX) * pZ;
+  H += (h2 * pY) * pT;
+  H -= ((h2 * P.l1) * pY) * pX;
+  H += ((1.0 - h2 * P.l2) * pY) * pY;
+  H -= ((h2 * P.l3) * pY) * pZ;
+  H += (h3 * pZ) * pT;
+  H -= ((h3 * P.l1) * pZ) * pX;
+  H -= ((h3 * P.l2) * pZ) * pY;
+  H += ((1.0 - h3 * P.l3) * pZ) * pZ;
+  return H;
+}
+
+// dX^i/dlambda at the centre (the rows of g^{ab} as ks_inv forms them).
+KT_HD void ks_rows(const KSPoint& P, double pT, double pX, double pY, double pZ, double k[3]) {
+  const double h1 = P.H * P.l1, h2 = P.H * P.l2, h3 = P.H * P.l3;
+  k[0] = (((0.0 + h1) * pT + (1.0 - h1 * P.l1) * pX) + (0.0 - h1 * P.l2) * pY) + (0.0 - h1 * P.l3) * pZ;
+  k[1] = (((0.0 + h2) * pT + (0.0 - h2 * P.l1) * pX) + (1.0 - h2 * P.l2) * pY) + (0.0 - h2 * P.l3) * pZ;
+  k[2] = (((0.0 + h3) * pT + (0.0 - h3 * P.l1) * pX) + (0.0 - h3 * P.l2) * pY) + (1.0 - h3 * P.l3) * pZ;
+}
+
+// A coordinate the quotients take: zero or of moderate size.
+KT_HD bool ks_coord_ok(double x) {
+  return is_zero(x) | ((hi_word(x) & 0x7fffffffu) - ((1023u - 200u) << 20) < (260u << 20));
+}
+
+// -(hp - hm)/(2 eps) from the two H without their 1/2.
+KT_HD double ks_slope(double d, double eps, uint32_t* top, bool* ok) {
+  const double e = 4.0 * eps;
+  *top |= top_ones(e);
+  *ok = *ok & (is_zero(d) | in_range(d, 400));
+  return -quot(d, make_rcp(e));
+}
+
+// k as ks_rhs; false (k not usable) where the caller has to take ks_rhs.
+// Bound by the FP64 pipe (150 instructions per point, 1050 per RHS, 77% of
+// the pipe's rate on the 1280 x 720 Kerr frame: 61 -> 51.6 ms).  The axes are
+// a rolled loop of two points each (53.2 ms unrolled, 55.7 with the six
+// points rolled: one point alone leaves the pipe waiting for its own results).
+KT_HD bool ks_rhs_exact(const Metric& g, double X, double Y, double Z, double pX, double pY,
+                        double pZ, double pT, double k[6]) {
+  const double eX = 1e-5 * (fabs(X) + 0.1);
+  const double eY = 1e-5 * (fabs(Y) + 0.1);
+  const double eZ = 1e-5 * (fabs(Z) + 0.1);
+  uint32_t top = 0;
+  bool ok = (g.tame != 0) & ks_coord_ok(X) & ks_coord_ok(Y) & ks_coord_ok(Z);
+  ks_rows(ks_point<true>(g, X, Y, Z, &top, &ok), pT, pX, pY, pZ, k);
+  KT_ROLLED
+  for (int i = 0; i < 3; ++i) {
+    const double e = i == 0 ? eX : i == 1 ? eY : eZ;
+    const double dx = i == 0 ? e : 0.0, dy = i == 1 ? e : 0.0, dz = i == 2 ? e : 0.0;
+    const double hp = ks_ham2(ks_point<false>(g, X + dx, Y + dy, Z + dz, &top, &ok), pT, pX, pY, pZ);
+    const double hm = ks_ham2(ks_point<false>(g, X - dx, Y - dy, Z - dz, &top, &ok), pT, pX, pY, pZ);
+    const double s = ks_slope(hp - hm, e, &top, &ok);
+    if (i == 0) k[3] = s;
+    else if (i == 1) k[4] = s;
+    else k[5] = s;
+  }
+  return ok & ((top & kTopBit) == 0u);
+}
+
+KT_HD_CALL void ks_rhs_rest(const Metric& g, double X, double Y, double Z, double pX, double pY,
+                            double pZ, double pT, double k[6]) {
+  ks_rhs(g, X, Y, Z, pX, pY, pZ, pT, k);
 }
 
 // BL_to_KS_spatial (knds_metric.hpp:368-387) from precomputed sin/cos.

@@ -62,4 +62,36 @@ long ec_bl_rhs(double M, double a, double Q, double L, int lam, long n, const do
   }
   return bad;
 }
+
+long ec_sqrt(long n, const double* x, long* refused) {
+  long bad = 0;
+  *refused = 0;
+  for (long i = 0; i < n; ++i) {
+    if (top_edge(x[i]) & kTopBit) {
+      ++*refused;
+      continue;
+    }
+    const double g = make_root(x[i]).g, e = sqrt(x[i]);
+    if (memcmp(&g, &e, 8) != 0) ++bad;
+  }
+  return bad;
+}
+
+// States (X, Y, Z, p_X, p_Y, p_Z, p_T) of the KS chart, as ec_bl_rhs.
+long ec_ks_rhs(double M, double a, double Q, long n, const double* y, long* refused) {
+  const Metric g = make_metric(M, a, Q, 0.0);
+  long bad = 0;
+  *refused = 0;
+  for (long i = 0; i < n; ++i) {
+    const double* s = y + 7 * i;
+    double k[6], e[6];
+    if (!ks_rhs_exact(g, s[0], s[1], s[2], s[3], s[4], s[5], s[6], k)) {
+      ++*refused;
+      continue;
+    }
+    ks_rhs(g, s[0], s[1], s[2], s[3], s[4], s[5], s[6], e);
+    if (memcmp(k, e, sizeof k) != 0) ++bad;
+  }
+  return bad;
+}
 }

@@ -28,6 +28,8 @@ def ec():
     L.ec_quot.argtypes, L.ec_quot.restype = [N, P, P, P], N
     L.ec_sincos.argtypes, L.ec_sincos.restype = [N, P, P], N
     L.ec_bl_rhs.argtypes, L.ec_bl_rhs.restype = [D, D, D, D, ctypes.c_int, N, P, P], N
+    L.ec_sqrt.argtypes, L.ec_sqrt.restype = [N, P, P], N
+    L.ec_ks_rhs.argtypes, L.ec_ks_rhs.restype = [D, D, D, N, P, P], N
     return L
 
 
@@ -106,3 +108,64 @@ def test_bl_rhs_exact_is_bl_rhs(ec, M, a, Q, L):
         tame = (a == 0.0 or abs(a) >= 2.0 ** -40) and (L == 0.0 or abs(L) >= 2.0 ** -90)
         # in range everywhere but at the states chosen to leave it
         assert refused.value < 0.05 * len(y) if tame else refused.value == len(y)
+
+
+def _hard_roots():
+    """x whose square root lies closest to a rounding midpoint: K^2 + D a
+    multiple of 2^52 (2^53), D = +-(K - j) or +-(K + j) with small even j, K a
+    53-bit integer (found bit by bit from the lowest)."""
+    out = []
+    for j in range(2, 200, 2):
+        for sg in (-1, 1):
+            for t in (-1, 1):
+                for mb in (52, 53):
+                    for k in (0, 1):
+                        for b in range(1, mb + 1):
+                            if (k * k + sg * (k + t * j)) % (1 << b):
+                                k |= 1 << (b - 1)
+                                if (k * k + sg * (k + t * j)) % (1 << b):
+                                    break
+                        else:
+                            for kk in (k, k + (1 << 52)):
+                                x = kk * kk + sg * (kk + t * j)
+                                if 1 << 52 <= kk < 1 << 53 and x > 0:
+                                    out.append(float(x >> 52))
+    return np.array(out)
+
+
+def test_roots_are_the_ieee_ones(ec):
+    rng = np.random.default_rng(6)
+    hard = _hard_roots()
+    g = np.ldexp(rng.integers(1 << 53, 1 << 54, 500_000).astype(np.float64), -53)
+    x = np.concatenate([np.abs(_bits(rng, 500_000, -250, 250)), g * g, hard, hard * 4.0, hard * 2.0,
+                        1.0 + np.arange(2000) * 2.0 ** -52, 4.0 - np.arange(2000) * 2.0 ** -51,
+                        np.arange(1.0, 2000.0) ** 2])
+    x = np.ascontiguousarray(x)
+    refused = ctypes.c_long()
+    assert len(hard) > 500
+    assert ec.ec_sqrt(len(x), _p(x), ctypes.byref(refused)) == 0
+    assert refused.value < 0.02 * len(x)
+
+
+@pytest.mark.parametrize("M,a,Q", [(1.0, 0.5, 0.0), (1.0, 0.998, 0.0), (1.0, 0.0, 0.0),
+                                   (1.0, -0.7, 0.3), (2.5, 1.1, 2.0), (1.0, 1e-14, 0.1)])
+def test_ks_rhs_exact_is_ks_rhs(ec, M, a, Q):
+    rng = np.random.default_rng(7)
+    n = 200_000
+    y = rng.uniform(-1, 1, (n, 7))
+    y[:, :3] *= np.exp(rng.uniform(-1, 5, n))[:, None]
+    y[:, 3:6] *= 2.0
+    y[:, 6] = -rng.uniform(0.5, 1.5, n)
+    q = n // 50
+    for i, c in enumerate((0, 1, 2, 4)):  # coordinate planes, signed zeros
+        y[i * q:(i + 1) * q, c] = np.where(rng.random(q) < 0.5, 0.0, -0.0)
+    y[4 * q:5 * q, 2] *= 1e-6
+    y[5 * q:6 * q, :2] *= 1e-6  # near the axis
+    y[-7:, 0] = [np.nan, np.inf, 1e300, 1e-300, -np.inf, 1e-160, 0.0]
+    y[-2:, 1:3] = 0.0
+    y[-12:-8, 3] = [np.nan, np.inf, 1e300, 1e-160]
+    y = np.ascontiguousarray(y)
+    refused = ctypes.c_long()
+    assert ec.ec_ks_rhs(M, a, Q, n, _p(y), ctypes.byref(refused)) == 0
+    tame = a == 0.0 or abs(a) >= 2.0 ** -40
+    assert refused.value < 0.05 * n if tame else refused.value == n
