@@ -27,6 +27,9 @@
 
 namespace kt {
 
+// h / 6 as the IEEE quotient (halving is exact).
+KT_HD double sixth(double h) { return 0.5 * ktm_div3(h); }
+
 enum : int { kOutEscaped = 0, kOutDisk = 1, kOutHorizon = 2 };
 enum : int { kStEvent = 0, kStStepCap = 1, kStRejectCap = 2, kStNonfinite = 3, kStCreep = 4 };
 enum : int { kEvNone = 0, kEvDisk = 1, kEvHorizon = 2, kEvEscape = 3 };
@@ -76,8 +79,11 @@ KT_HD int doubling_update(double err, double tol, double* dlam) {
     return -1;
   }
   const int accepted = (err < tol || *dlam < 1e-10);
+  // one pow for both outcomes, so that a warp with lanes of both runs it once
+  double p = 0.0;
+  if (!accepted || err > 1e-14) p = pow_ctl(tol / err, accepted ? 0.2 : 0.25);
   if (accepted) {
-    const double scale = (err > 1e-14) ? 0.9 * ktm_pow(tol / err, 0.2) : 4.0;
+    const double scale = (err > 1e-14) ? 0.9 * p : 4.0;
     double hnew = *dlam * scale;
     if (!finite(hnew)) hnew = *dlam;
     *dlam = hnew;
@@ -85,7 +91,7 @@ KT_HD int doubling_update(double err, double tol, double* dlam) {
     if (*dlam < 1e-10) *dlam = 1e-10;
   } else {
     const double half = *dlam * 0.5;
-    double hnew = (*dlam * 0.9) * ktm_pow(tol / err, 0.25);
+    double hnew = (*dlam * 0.9) * p;
     if (!finite(hnew)) hnew = half;
     *dlam = hnew;
     if (*dlam > half) *dlam = half;
@@ -292,7 +298,7 @@ struct BLRk4 : BLBase {
         for (int i = 0; i < 4; ++i) kp[i] = k[i];
         return false;
       case 2: {
-        const double w = h / 6.0;
+        const double w = sixth(h);
         A[0] = r + w * (sum[0] + k[0]);
         A[1] = th + w * (sum[1] + k[1]);
         A[2] = pr + w * (sum[2] + k[2]);
@@ -300,7 +306,7 @@ struct BLRk4 : BLBase {
         return false;
       }
       case 5: {
-        const double w = (0.5 * h) / 6.0;
+        const double w = sixth(0.5 * h);
         B1[0] = r + w * (sum[0] + k[0]);
         B1[1] = th + w * (sum[1] + k[1]);
         B1[2] = ph + w * (sum[4] + k[4]);
@@ -309,7 +315,7 @@ struct BLRk4 : BLBase {
         return false;
       }
       default: {  // 9: path B2 done -> error control
-        const double w = (0.5 * h) / 6.0;
+        const double w = sixth(0.5 * h);
         const double Br = B1[0] + w * (sum[0] + k[0]);
         const double Bth = B1[1] + w * (sum[1] + k[1]);
         const double Bph = B1[2] + w * (sum[4] + k[4]);
@@ -346,6 +352,19 @@ struct BLRk4 : BLBase {
   }
 };
 
+// The Dormand-Prince tableau: stages 2..6, the fifth- and fourth-order weights.
+#define KT_DP_A2 {1.0 / 5.0}
+#define KT_DP_A3 {3.0 / 40.0, 9.0 / 40.0}
+#define KT_DP_A4 {44.0 / 45.0, -56.0 / 15.0, 32.0 / 9.0}
+#define KT_DP_A5 {19372.0 / 6561.0, -25360.0 / 2187.0, 64448.0 / 6561.0, -212.0 / 729.0}
+#define KT_DP_A6 \
+  {9017.0 / 3168.0, -355.0 / 33.0, 46732.0 / 5247.0, 49.0 / 176.0, -5103.0 / 18656.0}
+#define KT_DP_B5 \
+  {35.0 / 384.0, 0.0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0, 11.0 / 84.0}
+#define KT_DP_B4                                                                    \
+  {5179.0 / 57600.0,    0.0,           7571.0 / 16695.0, 393.0 / 640.0,             \
+   -92097.0 / 339200.0, 187.0 / 2100.0, 1.0 / 40.0}
+
 // DOPRI5 (dopri5_adaptive, geodesic.hpp:284-414), kSlots = 6: slots 0..4
 // -> k2..k6, slot 5 -> k7 = f(y5) then error control.  FSAL: after an
 // accepted step k1 = k7, so only a new ray needs slot -1.  Phi is not
@@ -356,12 +375,39 @@ struct BLDopri5 : BLBase {
 
   KT_HD void init(const Frame& f, const Geo& s) { init_state(f, s); }
 
+  // Step-size update for the error norm err; true: the step is accepted.
+  KT_HD static bool control(double err, double* h) {
+    if (!finite(err)) {
+      *h = (finite(*h) && *h > 1e-10) ? *h * 0.5 : 1e-6;
+      if (*h < 1e-10) *h = 1e-10;
+      return false;
+    }
+    const bool accepted = err <= 1.0 || *h < 1e-10;
+    double p = 0.0;  // one pow for both outcomes, as in doubling_update
+    if (!accepted || err > 1e-12) p = pow_ctl(1.0 / err, accepted ? 0.2 : 0.25);
+    if (accepted) {
+      const double fac = (err > 1e-12) ? 0.9 * p : 4.0;
+      double hnew = *h * fac;
+      if (!finite(hnew)) hnew = *h;
+      if (hnew > 100.0) hnew = 100.0;
+      if (hnew < 1e-10) hnew = 1e-10;
+      *h = hnew;
+      return true;
+    }
+    double hnew = (*h * 0.9) * p;
+    if (!finite(hnew)) hnew = *h * 0.5;
+    *h = dmax(hnew, 1e-10);
+    return false;
+  }
+
   // advance (geodesic.hpp:300-310): y = s + sum_i (h w_i) k_i, in order.
   template <int N>
   KT_HD void adv(const double* w, double y[4]) const {
     y[0] = r; y[1] = th; y[2] = pr; y[3] = pth;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
+      // a zero weight (k2 in both results) adds a zero
+      if (w[i] == 0.0) continue;
       const double hw = h * w[i];
       y[0] += hw * kk[i][0];
       y[1] += hw * kk[i][1];
@@ -370,22 +416,19 @@ struct BLDopri5 : BLBase {
     }
   }
 
-  KT_HD void input(int slot, double y[4]) const {
-    const double a2[1] = {1.0 / 5.0};
-    const double a3[2] = {3.0 / 40.0, 9.0 / 40.0};
-    const double a4[3] = {44.0 / 45.0, -56.0 / 15.0, 32.0 / 9.0};
-    const double a5[4] = {19372.0 / 6561.0, -25360.0 / 2187.0, 64448.0 / 6561.0, -212.0 / 729.0};
-    const double a6[5] = {9017.0 / 3168.0, -355.0 / 33.0, 46732.0 / 5247.0, 49.0 / 176.0,
-                          -5103.0 / 18656.0};
-    const double b5[6] = {35.0 / 384.0, 0.0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0,
-                          11.0 / 84.0};
+  KT_HD void input(int slot, double y[4]) {
+    const double a2[1] = KT_DP_A2, a3[2] = KT_DP_A3, a4[3] = KT_DP_A4, a5[4] = KT_DP_A5;
+    const double a6[5] = KT_DP_A6, b5[6] = KT_DP_B5;
     switch (slot) {
       case 0: adv<1>(a2, y); break;
       case 1: adv<2>(a3, y); break;
       case 2: adv<3>(a4, y); break;
       case 3: adv<4>(a5, y); break;
       case 4: adv<5>(a6, y); break;
-      case 5: adv<6>(b5, y); break;
+      case 5:
+        adv<6>(b5, y);
+        for (int i = 0; i < 4; ++i) kk[1][i] = y[i];  // the fifth-order result; k2 is done with
+        break;
       default: y[0] = r; y[1] = th; y[2] = pr; y[3] = pth; break;
     }
   }
@@ -404,12 +447,9 @@ struct BLDopri5 : BLBase {
       default: break;
     }
     for (int i = 0; i < 4; ++i) kk[6][i] = k[i];
-    const double b5[6] = {35.0 / 384.0, 0.0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0,
-                          11.0 / 84.0};
-    const double b4[7] = {5179.0 / 57600.0, 0.0, 7571.0 / 16695.0, 393.0 / 640.0,
-                          -92097.0 / 339200.0, 187.0 / 2100.0, 1.0 / 40.0};
+    const double b4[7] = KT_DP_B4;
     double y5[4], y4[4];
-    adv<6>(b5, y5);
+    for (int i = 0; i < 4; ++i) y5[i] = kk[1][i];
     adv<7>(b4, y4);
     const double ref[4] = {r, th, pr, pth};
     double err2 = 0.0;
@@ -420,16 +460,7 @@ struct BLDopri5 : BLBase {
     const double err = sqrt(err2 / 4.0);
     step_used = h;
     ++attempts;
-    if (!finite(err)) {
-      h = (finite(h) && h > 1e-10) ? h * 0.5 : 1e-6;
-      if (h < 1e-10) h = 1e-10;
-    } else if (err <= 1.0 || h < 1e-10) {
-      const double fac = (err > 1e-12) ? 0.9 * ktm_pow(1.0 / err, 0.2) : 4.0;
-      double hnew = h * fac;
-      if (!finite(hnew)) hnew = h;
-      if (hnew > 100.0) hnew = 100.0;
-      if (hnew < 1e-10) hnew = 1e-10;
-      h = hnew;
+    if (control(err, &h)) {
       const double sp_r = r, sp_th = th;
       const double k0_r = kk[0][0], k0_th = kk[0][1];
       r = y5[0];
@@ -439,10 +470,6 @@ struct BLDopri5 : BLBase {
       for (int i = 0; i < 4; ++i) kk[0][i] = kk[6][i];  // FSAL
       if (events(f, sp_r, sp_th, ph, k0_r, k0_th, kk[0][0], kk[0][1], o)) return true;
       return next_step(f, o);
-    } else {
-      double hnew = (h * 0.9) * ktm_pow(1.0 / err, 0.25);
-      if (!finite(hnew)) hnew = h * 0.5;
-      h = dmax(hnew, 1e-10);
     }
     int st;
     if (reject_cap(h, &rejects, &st)) {
@@ -608,17 +635,17 @@ struct KSRk4 {
         }
         return false;
       case 2: {
-        const double w = h / 6.0;
+        const double w = sixth(h);
         for (int i = 0; i < 6; ++i) A[i] = s[i] + w * (sum[i] + k[i]);
         return false;
       }
       case 5: {
-        const double w = (0.5 * h) / 6.0;
+        const double w = sixth(0.5 * h);
         for (int i = 0; i < 6; ++i) B1[i] = s[i] + w * (sum[i] + k[i]);
         return false;
       }
       default: {  // 9
-        const double w = (0.5 * h) / 6.0;
+        const double w = sixth(0.5 * h);
         double B[6];
         for (int i = 0; i < 6; ++i) B[i] = B1[i] + w * (sum[i] + k[i]);
         const double e0 = A[0] - B[0], e1 = A[1] - B[1], ez = A[2] - B[2];
@@ -900,7 +927,7 @@ struct Bundle {
         for (int i = 0; i < 8; ++i) kpW[i] = kW[i];
         return false;
       case 2: {
-        const double w = h / 6.0;
+        const double w = sixth(h);
         A[0] = r + w * (sum[0] + k[0]);
         A[1] = th + w * (sum[1] + k[1]);
         A[2] = pr + w * (sum[2] + k[2]);
@@ -908,7 +935,7 @@ struct Bundle {
         return false;
       }
       case 5: {
-        const double w = (0.5 * h) / 6.0;
+        const double w = sixth(0.5 * h);
         B1[0] = r + w * (sum[0] + k[0]);
         B1[1] = th + w * (sum[1] + k[1]);
         B1[2] = ph + w * (sum[4] + k[4]);
@@ -918,7 +945,7 @@ struct Bundle {
         return false;
       }
       default: {  // 9
-        const double w = (0.5 * h) / 6.0;
+        const double w = sixth(0.5 * h);
         const double Br = B1[0] + w * (sum[0] + k[0]);
         const double Bth = B1[1] + w * (sum[1] + k[1]);
         const double Bph = B1[2] + w * (sum[4] + k[4]);
@@ -1262,7 +1289,7 @@ struct SepRk4 {
         for (int i = 0; i < 2; ++i) kp[i] = k[i];
         return false;
       case 2: {
-        const double w = h / 6.0;
+        const double w = sixth(h);
         A[0] = r + w * (sum[0] + k[0]);
         A[1] = th + w * (sum[1] + k[1]);
         A[2] = ph + w * (sum[2] + k[2]);
@@ -1270,7 +1297,7 @@ struct SepRk4 {
         return false;
       }
       case 5: {
-        const double w = (0.5 * h) / 6.0;
+        const double w = sixth(0.5 * h);
         B1[0] = r + w * (sum[0] + k[0]);
         B1[1] = th + w * (sum[1] + k[1]);
         B1[2] = ph + w * (sum[2] + k[2]);
@@ -1278,7 +1305,7 @@ struct SepRk4 {
         return false;
       }
       default: {  // 9: path B2 done -> error control
-        const double w = (0.5 * h) / 6.0;
+        const double w = sixth(0.5 * h);
         const double Br = B1[0] + w * (sum[0] + k[0]);
         const double Bth = B1[1] + w * (sum[1] + k[1]);
         const double Bph = B1[2] + w * (sum[2] + k[2]);

@@ -277,13 +277,19 @@ KTM_FN double ktm_div3(double x) { return ktm_div_odd(x, 3.0, 0x1.5555555555555p
 
 /* -------------------------------------------------------------------- exp */
 
-/* exp(hi + lo) where |lo| <= ulp(hi). */
-KTM_FN double ktm_exp_dd(double hi, double lo) {
-  if (ktm_isnan(hi)) return hi;
-  if (hi > 709.8) return ktm_inf();
-  if (hi < -745.2) return 0.0;
+/* exp(hi + lo) 2^-k for |hi| < 746, |lo| <= ulp(hi); k out. */
+#if defined(__CUDACC__)
+static __constant__ double ktm_exp_c[13] = KTM_EXP_COEFFS;
+#endif
+KTM_FN double ktm_exp_core(double hi, double lo, int* ke) {
+#if defined(__CUDA_ARCH__)
+  const double* c = ktm_exp_c;
+#else
   const double c[13] = KTM_EXP_COEFFS;
-  const double k = rint(hi * KTM_INV_LN2);
+#endif
+  const double kMagic = 0x1.8p52; /* rint() by adding and subtracting 1.5 2^52 */
+  const double kt = KTM_ADD_RN(KTM_MUL_RN(hi, KTM_INV_LN2), kMagic);
+  const double k = KTM_ADD_RN(kt, -kMagic);
   double r = fma(-k, KTM_LN2_HI, hi);
   r = fma(-k, KTM_LN2_LO, r);
   r = r + lo;
@@ -300,37 +306,34 @@ KTM_FN double ktm_exp_dd(double hi, double lo) {
   p = fma(p, r, c[2]);
   p = fma(p, r, c[1]);
   p = fma(p, r, c[0]);
-  const double e = 1.0 + fma(r * r, p, r);
-  return ktm_scale(e, (int)k);
+  *ke = (int)(uint32_t)ktm_bits(kt);
+  return 1.0 + fma(r * r, p, r);
+}
+
+/* exp(hi + lo) where |lo| <= ulp(hi). */
+KTM_FN double ktm_exp_dd(double hi, double lo) {
+  if (ktm_isnan(hi)) return hi;
+  if (hi > 709.8) return ktm_inf();
+  if (hi < -745.2) return 0.0;
+  int k;
+  const double e = ktm_exp_core(hi, lo, &k);
+  return ktm_scale(e, k);
 }
 
 KTM_FN double ktm_exp(double x) { return ktm_exp_dd(x, 0.0); }
 
 /* -------------------------------------------------------------------- log */
 
-/* log(x) as a double-double for finite x > 0. */
-KTM_FN void ktm_log_dd(double x, double* out_hi, double* out_lo) {
+/* log(2^e (1 + s)/(1 - s)) as a double-double, s + s_lo the double-double quotient. */
+#if defined(__CUDACC__)
+static __constant__ double ktm_log_c[12] = KTM_LOG_COEFFS;
+#endif
+KTM_FN void ktm_log_finish(double s, double s_lo, int e, double* out_hi, double* out_lo) {
+#if defined(__CUDA_ARCH__)
+  const double* lc = ktm_log_c;
+#else
   const double lc[12] = KTM_LOG_COEFFS;
-  int e = 0;
-  if (x < 0x1p-1022) {
-    x *= 0x1p54;
-    e = -54;
-  }
-  uint64_t u = ktm_bits(x);
-  e += (int)((u >> 52) & 0x7ff) - 1023;
-  u = (u & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL;
-  double m = ktm_from_bits(u);
-  if (m > 2.0 * KTM_SQRT2_OVER_2) {
-    m *= 0.5;
-    e += 1;
-  }
-  const double f = m - 1.0;                 /* exact (Sterbenz) */
-  const double den = 2.0 + f;
-  const double den_lo = (2.0 - den) + f;    /* Fast2Sum, |f| < 2 */
-  const double s = f / den;
-  double rem = fma(-s, den, f);
-  rem = rem - s * den_lo;
-  const double s_lo = rem / den;
+#endif
   const double z = s * s;
   double p = lc[11];
   p = fma(p, z, lc[10]);
@@ -357,6 +360,31 @@ KTM_FN void ktm_log_dd(double x, double* out_hi, double* out_lo) {
   const double hi = sum + lo;
   *out_hi = hi;
   *out_lo = (sum - hi) + lo;
+}
+
+/* log(x) as a double-double for finite x > 0. */
+KTM_FN void ktm_log_dd(double x, double* out_hi, double* out_lo) {
+  int e = 0;
+  if (x < 0x1p-1022) {
+    x *= 0x1p54;
+    e = -54;
+  }
+  uint64_t u = ktm_bits(x);
+  e += (int)((u >> 52) & 0x7ff) - 1023;
+  u = (u & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL;
+  double m = ktm_from_bits(u);
+  if (m > 2.0 * KTM_SQRT2_OVER_2) {
+    m *= 0.5;
+    e += 1;
+  }
+  const double f = m - 1.0;                 /* exact (Sterbenz) */
+  const double den = 2.0 + f;
+  const double den_lo = (2.0 - den) + f;    /* Fast2Sum, |f| < 2 */
+  const double s = f / den;
+  double rem = fma(-s, den, f);
+  rem = rem - s * den_lo;
+  const double s_lo = rem / den;
+  ktm_log_finish(s, s_lo, e, out_hi, out_lo);
 }
 
 KTM_FN double ktm_log(double x) {

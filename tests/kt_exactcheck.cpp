@@ -94,4 +94,40 @@ long ec_ks_rhs(double M, double a, double Q, long n, const double* y, long* refu
   }
   return bad;
 }
+
+// pow_ctl against ktm_pow for the controllers' exponents.
+long ec_pow(long n, const double* x) {
+  long bad = 0;
+  for (long i = 0; i < n; ++i)
+    for (int j = 0; j < 2; ++j) {
+      const double y = j ? 0.25 : 0.2, p = pow_ctl(x[i], y), e = ktm_pow(x[i], y);
+      if (memcmp(&p, &e, 8) != 0) ++bad;
+    }
+  return bad;
+}
+
+// first_event's quick test: of n cubics (y0, y1, dy0, dy1, h, target), those
+// it dismisses although the search (without the test) finds an event;
+// *quick counts the dismissed, *none those without an event.
+long ec_no_event(long n, const double* v, long* quick, long* none) {
+  long bad = 0;
+  *quick = *none = 0;
+  for (long i = 0; i < n; ++i) {
+    const double *c = v + 6 * i, target = c[5];
+    bool found = false;
+    double f0 = c[0] - target;
+    found = fabs(f0) <= 1e-12;
+    for (int b = 1; b <= 8 && !found; ++b) {
+      const double f1 =
+          (b == 8) ? (c[1] - target) : (hermite(c[0], c[1], c[2], c[3], c[4], b / 8.0) - target);
+      found = fabs(f1) <= 1e-12 || sign_change(f0, f1);
+      f0 = f1;
+    }
+    const bool no = no_event(c[0], c[1], c[2], c[3], c[4], target);
+    *quick += no;
+    *none += !found;
+    if (no && found) ++bad;
+  }
+  return bad;
+}
 }

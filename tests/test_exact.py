@@ -29,6 +29,8 @@ def ec():
     L.ec_sincos.argtypes, L.ec_sincos.restype = [N, P, P], N
     L.ec_bl_rhs.argtypes, L.ec_bl_rhs.restype = [D, D, D, D, ctypes.c_int, N, P, P], N
     L.ec_sqrt.argtypes, L.ec_sqrt.restype = [N, P, P], N
+    L.ec_pow.argtypes, L.ec_pow.restype = [N, P], N
+    L.ec_no_event.argtypes, L.ec_no_event.restype = [N, P, P, P], N
     L.ec_ks_rhs.argtypes, L.ec_ks_rhs.restype = [D, D, D, N, P, P], N
     return L
 
@@ -169,3 +171,34 @@ def test_ks_rhs_exact_is_ks_rhs(ec, M, a, Q):
     assert ec.ec_ks_rhs(M, a, Q, n, _p(y), ctypes.byref(refused)) == 0
     tame = a == 0.0 or abs(a) >= 2.0 ** -40
     assert refused.value < 0.05 * n if tame else refused.value == n
+
+
+def test_controller_pow_is_pow(ec):
+    rng = np.random.default_rng(8)
+    x = np.concatenate([rng.uniform(0.5, 2.0, 300_000), np.abs(_bits(rng, 300_000, -1022, 1024)),
+                        1.0 + np.arange(-2000, 2000) * 2.0 ** -52, np.sqrt(0.5) + np.arange(-50, 50) * 2.0 ** -53,
+                        np.array([0.0, -0.0, -1.0, np.inf, np.nan, 5e-324, 2.0 ** -1022, 1.0, 1.7e308]),
+                        np.ldexp(1.0, np.arange(-1000, 1000))])
+    assert ec.ec_pow(len(x), _p(np.ascontiguousarray(x))) == 0
+
+
+@pytest.mark.parametrize("target", [np.pi / 2, 0.0])
+def test_quick_event_test_dismisses_no_event(ec, target):
+    rng = np.random.default_rng(9)
+    n = 1_000_000
+    s = np.exp(rng.uniform(-30, 1, n))  # distance from the target, down to rounding
+    v = np.empty((n, 6))
+    v[:, 4] = np.exp(rng.uniform(-20, 4.6, n))
+    for i in (0, 1):
+        v[:, i] = target + rng.uniform(-1, 1, n) * s
+        v[:, 2 + i] = rng.uniform(-2, 2, n) * s / v[:, 4] * np.exp(rng.uniform(-3, 1.5, n))
+    v[:, 5] = target
+    v[:100, 0] = target
+    v[100:200, 1] = target
+    v[200:300, 2] = np.nan
+    v[300:400, 3] = np.inf
+    q = n // 4  # both ends on one side, as between crossings
+    v[-q:, 1] = target + np.abs(v[-q:, 1] - target) * np.sign(v[-q:, 0] - target)
+    quick, none = ctypes.c_long(), ctypes.c_long()
+    assert ec.ec_no_event(n, _p(np.ascontiguousarray(v)), ctypes.byref(quick), ctypes.byref(none)) == 0
+    assert quick.value > 0.5 * none.value  # it is worth its place
