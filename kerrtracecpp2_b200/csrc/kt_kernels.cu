@@ -73,24 +73,43 @@ struct ModeBundle {
 };
 
 // Bundles with two lanes per ray (k_trace_pair): the right-hand side is
-// split by bundle_rhs_half, the halves swapped with one shuffle each, and
-// bundle_rhs_combine assembles it in bundle_rhs's order (bit-identical); the
+// split by bundle_half_exact, the halves swapped with one shuffle each, and
+// bundle_combine_exact assembles it in bundle_rhs's order (bit-identical); the
 // even lane runs the machine's bookkeeping.
-__device__ __forceinline__ void bundle_rhs_paired(const Metric& g, const double y[4], double pt,
-                                                  double pphi, const double W[8], double k[5],
-                                                  double kW[8], bool odd, unsigned pmask) {
-  BundleHalf me, other;
-  bundle_rhs_half(g, y[0], y[1], y[2], y[3], pt, pphi, odd, &me);
+__device__ __forceinline__ void swap_halves(unsigned mask, const BundleHalf& me, BundleHalf* other) {
 #pragma unroll
   for (int t = 0; t < 3; ++t)
 #pragma unroll
-    for (int j = 0; j < 5; ++j) other.h5[t][j] = __shfl_xor_sync(pmask, me.h5[t][j], 1);
+    for (int j = 0; j < 5; ++j) other->h5[t][j] = __shfl_xor_sync(mask, me.h5[t][j], 1);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) other.h1[i] = __shfl_xor_sync(pmask, me.h1[i], 1);
+  for (int i = 0; i < 4; ++i) other->h1[i] = __shfl_xor_sync(mask, me.h1[i], 1);
+}
+
+// The general form, for the states the exact quotients do not take; both
+// lanes of the pair (mask) call it together.
+__device__ __noinline__ void bundle_rhs_pair_rest(const Metric& g, const double y[4], double pt,
+                                                  double pphi, const double W[8], double k[5],
+                                                  double kW[8], bool odd, unsigned mask) {
+  BundleHalf me, other;
+  bundle_rhs_half(g, y[0], y[1], y[2], y[3], pt, pphi, odd, &me);
+  swap_halves(mask, me, &other);
   // the even lane's view (the odd lane's result is not used)
   bundle_rhs_combine(me, other, y[0], y[2], y[3], W, k, kW);
 }
 
+template <bool kLam>
+__device__ __forceinline__ void bundle_rhs_paired(const Metric& g, const double y[4], double pt,
+                                                  double pphi, const double W[8], double k[5],
+                                                  double kW[8], bool odd, unsigned pmask) {
+  BundleHalf me, other;
+  bool ok = bundle_half_exact<kLam>(g, y[0], y[1], y[2], y[3], pt, pphi, odd, &me);
+  swap_halves(pmask, me, &other);
+  ok = bundle_combine_exact(me, other, y[0], y[2], y[3], W, k, kW) & ok;
+  const unsigned pair = 3u << (threadIdx.x & 30u);
+  if (!__all_sync(pair, ok)) bundle_rhs_pair_rest(g, y, pt, pphi, W, k, kW, odd, pair);
+}
+
+template <bool kLam>
 struct ModeBundlePair {
   using Machine = Bundle;
   static constexpr int kSlots = Bundle::kSlots;
@@ -104,7 +123,7 @@ struct ModeBundlePair {
                                        unsigned pmask) {
     double y[4], yW[8], k[5], kW[8];
     m->input(s, y, yW);
-    bundle_rhs_paired(f.g, y, m->pt, m->pphi, yW, k, kW, odd, pmask);
+    bundle_rhs_paired<kLam>(f.g, y, m->pt, m->pphi, yW, k, kW, odd, pmask);
     __syncwarp(pmask);  // both lanes have read the record
     int done = 0;
     if (!odd) done = m->consume(f, s, k, kW, res) ? 1 : 0;
@@ -178,7 +197,7 @@ template <> struct Shape<struct ModeBundle> { static constexpr int kBlock = 128,
 #ifndef KT_BUNDLE_PAIR_REFILL
 #define KT_BUNDLE_PAIR_REFILL 8
 #endif
-template <> struct Shape<ModeBundlePair> {
+template <bool kLam> struct Shape<ModeBundlePair<kLam>> {
   static constexpr int kBlock = KT_BUNDLE_PAIR_BLOCK, kMinBlocks = KT_BUNDLE_PAIR_MINB,
                        kRefill = KT_BUNDLE_PAIR_REFILL;
 };
@@ -191,13 +210,21 @@ static cudaError_t launch_one(const Frame& f, const OutSoA& out, const RayList& 
   return cudaGetLastError();
 }
 
+template <class ModeT>
+static cudaError_t launch_pair(const Frame& f, const OutSoA& out, const RayList& rl,
+                               uint32_t* queue, const Fallback& fb, const LaunchShape& s,
+                               cudaStream_t stream) {
+  k_trace_pair<ModeT><<<s.grid, s.block, s.smem, stream>>>(f, out, rl, queue, fb);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_shape(Mode mode, int device, LaunchShape* shape) {
   if (is_mixed_mode(mode)) return launch_shape_mixed(mode, device, shape);
   switch (mode) {
     case kModeBLRk4: return shape_for_both<ModeBLRk4<true>, ModeBLRk4<false>>(device, shape);
     case kModeBLDopri5: return shape_for_both<ModeBLDopri5<true>, ModeBLDopri5<false>>(device, shape);
     case kModeKSRk4: return shape_for<ModeKSRk4>(device, shape);
-    case kModeBundle: return shape_for_pair<ModeBundlePair>(device, shape);
+    case kModeBundle: return shape_for_pair<ModeBundlePair<true>, ModeBundlePair<false>>(device, shape);
     case kModeSepRk4: return shape_for<ModeSepRk4>(device, shape);
     default: return cudaErrorInvalidValue;
   }
@@ -216,11 +243,12 @@ cudaError_t launch_trace(Mode mode, const Frame& f, const OutSoA& out, const Ray
       return lam ? launch_one<ModeBLDopri5<true>>(f, out, rl, queue, fb, s, stream)
                  : launch_one<ModeBLDopri5<false>>(f, out, rl, queue, fb, s, stream);
     case kModeKSRk4: return launch_one<ModeKSRk4>(f, out, rl, queue, fb, s, stream);
-    case kModeBundle: k_trace_pair<ModeBundlePair><<<s.grid, s.block, s.smem, stream>>>(f, out, rl, queue, fb); break;
+    case kModeBundle:
+      return lam ? launch_pair<ModeBundlePair<true>>(f, out, rl, queue, fb, s, stream)
+                 : launch_pair<ModeBundlePair<false>>(f, out, rl, queue, fb, s, stream);
     case kModeSepRk4: return launch_one<ModeSepRk4>(f, out, rl, queue, fb, s, stream);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 cudaError_t batch_shape(Mode mode, int variant, int device, LaunchShape* shape) {
@@ -231,7 +259,8 @@ cudaError_t batch_shape(Mode mode, int variant, int device, LaunchShape* shape) 
     case kModeKSRk4: return batch_shape<ModeKSRk4>(variant, device, shape);
     case kModeBundle:
       if (variant == kBatchPairVariant)
-        return batch_shape_pair_for<ModeBundlePair, kBatchBlock[kBatchPairVariant],
+        return batch_shape_pair_for<ModeBundlePair<true>, ModeBundlePair<false>,
+                                    kBatchBlock[kBatchPairVariant],
                                     kBatchMinBlocks[kBatchPairVariant]>(device, shape);
       return batch_shape<ModeBundle>(variant, device, shape);
     case kModeSepRk4: return batch_shape<ModeSepRk4>(variant, device, shape);
@@ -251,9 +280,11 @@ cudaError_t launch_batch(Mode mode, int variant, const BatchRays& br, uint32_t* 
     case kModeKSRk4: return batch_launch<ModeKSRk4>(variant, br, queue, fb, s, st);
     case kModeBundle:
       if (variant == kBatchPairVariant) {
-        k_trace_batch_pair<ModeBundlePair, kBatchBlock[kBatchPairVariant],
-                           kBatchMinBlocks[kBatchPairVariant]><<<s.grid, s.block, s.smem, st>>>(
-            br, queue, fb);
+        constexpr int kB = kBatchBlock[kBatchPairVariant], kM = kBatchMinBlocks[kBatchPairVariant];
+        if (br.lam)
+          k_trace_batch_pair<ModeBundlePair<true>, kB, kM><<<s.grid, s.block, s.smem, st>>>(br, queue, fb);
+        else
+          k_trace_batch_pair<ModeBundlePair<false>, kB, kM><<<s.grid, s.block, s.smem, st>>>(br, queue, fb);
         return cudaGetLastError();
       }
       return batch_launch<ModeBundle>(variant, br, queue, fb, s, st);

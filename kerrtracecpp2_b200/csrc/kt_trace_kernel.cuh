@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(Shape<ModeT>::kBlock, Shape<ModeT>::kMinBlocks
 }
 
 template <class ModeT>
-static cudaError_t shape_for_pair(int device, LaunchShape* shape) {
+static cudaError_t shape_for_pair_one(int device, LaunchShape* shape) {
   int sms = 0, per_sm = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
@@ -248,6 +248,15 @@ static cudaError_t shape_for_both(int device, LaunchShape* shape) {
   LaunchShape b;
   cudaError_t e = shape_for<A>(device, shape);
   if (e == cudaSuccess) e = shape_for<B>(device, &b);
+  if (e == cudaSuccess && b.grid > shape->grid) shape->grid = b.grid;
+  return e;
+}
+
+template <class A, class B>
+static cudaError_t shape_for_pair(int device, LaunchShape* shape) {
+  LaunchShape b;
+  cudaError_t e = shape_for_pair_one<A>(device, shape);
+  if (e == cudaSuccess) e = shape_for_pair_one<B>(device, &b);
   if (e == cudaSuccess && b.grid > shape->grid) shape->grid = b.grid;
   return e;
 }
@@ -389,7 +398,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
 }
 
 template <class ModeT, int BLOCK, int MINB>
-static cudaError_t batch_shape_pair_for(int device, LaunchShape* shape) {
+static cudaError_t batch_shape_pair_one(int device, LaunchShape* shape) {
   int sms = 0, per_sm = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
@@ -405,6 +414,15 @@ static cudaError_t batch_shape_pair_for(int device, LaunchShape* shape) {
   shape->grid = sms * per_sm;
   shape->smem = smem;
   return cudaSuccess;
+}
+
+template <class A, class B, int BLOCK, int MINB>
+static cudaError_t batch_shape_pair_for(int device, LaunchShape* shape) {
+  LaunchShape b;
+  cudaError_t e = batch_shape_pair_one<A, BLOCK, MINB>(device, shape);
+  if (e == cudaSuccess) e = batch_shape_pair_one<B, BLOCK, MINB>(device, &b);
+  if (e == cudaSuccess && b.grid > shape->grid) shape->grid = b.grid;
+  return e;
 }
 
 template <class ModeT, int BLOCK, int MINB>

@@ -130,4 +130,31 @@ long ec_no_event(long n, const double* v, long* quick, long* none) {
   }
   return bad;
 }
+
+// States (r, theta, p_r, p_theta, p_t, p_phi, W[8]) of the bundle right-hand
+// side split over two lanes (bundle_half_exact, bundle_combine_exact) against
+// bundle_rhs.
+long ec_bundle_rhs(double M, double a, double Q, double L, int lam, long n, const double* y,
+                   long* refused) {
+  const Metric g = make_metric(M, a, Q, L);
+  long bad = 0;
+  *refused = 0;
+  for (long i = 0; i < n; ++i) {
+    const double *s = y + 14 * i, *W = s + 6;
+    BundleHalf H[2];
+    bool ok = true;
+    for (int o = 0; o < 2; ++o)
+      ok = (lam ? bundle_half_exact<true>(g, s[0], s[1], s[2], s[3], s[4], s[5], o != 0, &H[o])
+                : bundle_half_exact<false>(g, s[0], s[1], s[2], s[3], s[4], s[5], o != 0, &H[o])) && ok;
+    double k[5], kW[8], e[5], eW[8];
+    ok = bundle_combine_exact(H[0], H[1], s[0], s[2], s[3], W, k, kW) && ok;
+    if (!ok) {
+      ++*refused;
+      continue;
+    }
+    bundle_rhs(g, s[0], s[1], s[2], s[3], s[4], s[5], W, e, eW);
+    if (memcmp(k, e, sizeof k) != 0 || memcmp(kW, eW, sizeof kW) != 0) ++bad;
+  }
+  return bad;
+}
 }

@@ -29,6 +29,7 @@ def ec():
     L.ec_sincos.argtypes, L.ec_sincos.restype = [N, P, P], N
     L.ec_bl_rhs.argtypes, L.ec_bl_rhs.restype = [D, D, D, D, ctypes.c_int, N, P, P], N
     L.ec_sqrt.argtypes, L.ec_sqrt.restype = [N, P, P], N
+    L.ec_bundle_rhs.argtypes, L.ec_bundle_rhs.restype = [D, D, D, D, ctypes.c_int, N, P, P], N
     L.ec_pow.argtypes, L.ec_pow.restype = [N, P], N
     L.ec_no_event.argtypes, L.ec_no_event.restype = [N, P, P, P], N
     L.ec_ks_rhs.argtypes, L.ec_ks_rhs.restype = [D, D, D, N, P, P], N
@@ -202,3 +203,17 @@ def test_quick_event_test_dismisses_no_event(ec, target):
     quick, none = ctypes.c_long(), ctypes.c_long()
     assert ec.ec_no_event(n, _p(np.ascontiguousarray(v)), ctypes.byref(quick), ctypes.byref(none)) == 0
     assert quick.value > 0.5 * none.value  # it is worth its place
+
+
+@pytest.mark.parametrize("M,a,Q,L", [(1.0, 0.998, 0.0, 0.0), (1.0, 0.0, 0.0, 0.0), (1.0, -0.7, 0.3, 0.0),
+                                     (1.0, 0.9, 0.2, 1e-5), (1.0, 0.5, 0.0, -1e-2), (1.0, 1e-14, 0.0, 0.0)])
+def test_split_bundle_rhs_exact_is_bundle_rhs(ec, M, a, Q, L):
+    rng = np.random.default_rng(10)
+    n = 100_000
+    y = np.ascontiguousarray(np.hstack([_states(rng, n), rng.uniform(-5, 5, (n, 8))]))
+    y[:100, 6:] = 0.0
+    for lam in ([1] if L != 0.0 else [0, 1]):
+        refused = ctypes.c_long()
+        assert ec.ec_bundle_rhs(M, a, Q, L, lam, n, _p(y), ctypes.byref(refused)) == 0
+        tame = a == 0.0 or abs(a) >= 2.0 ** -40
+        assert refused.value < 0.05 * n if tame else refused.value == n
