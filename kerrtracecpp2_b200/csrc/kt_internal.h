@@ -80,6 +80,7 @@ struct LaunchShape {
   int block;    // threads per block
   int grid;     // persistent blocks
   size_t smem;  // dynamic shared memory per block (ray machines)
+  int sms;      // multiprocessors of the device
 };
 
 // Occupancy-derived persistent grid for one mode (cached per device).

@@ -3,6 +3,7 @@
 // Compiled with --fmad=false: every multiply and add of the reference's
 // arithmetic is rounded separately, as in the reference's CPU build.
 #include "kt_elliptic.cuh"
+#include "kt_group.cuh"
 #include "kt_trace_kernel.cuh"
 
 namespace kt {
@@ -242,7 +243,14 @@ cudaError_t launch_trace(Mode mode, const Frame& f, const OutSoA& out, const Ray
     case kModeBLDopri5:
       return lam ? launch_one<ModeBLDopri5<true>>(f, out, rl, queue, fb, s, stream)
                  : launch_one<ModeBLDopri5<false>>(f, out, rl, queue, fb, s, stream);
-    case kModeKSRk4: return launch_one<ModeKSRk4>(f, out, rl, queue, fb, s, stream);
+    case kModeKSRk4:
+      // several lanes per ray where the rays do not fill the device
+      // (kt_group.cuh); a count on the device is not known here
+      if (!rl.n_dev && rl.n > 0 && rl.n <= kKs8MaxRays)
+        return launch_group<GroupKSRk4<8>>(f, out, rl, queue, fb, s.sms, stream);
+      if (!rl.n_dev && rl.n > 0 && rl.n <= kKs4MaxRays)
+        return launch_group<GroupKSRk4<4>>(f, out, rl, queue, fb, s.sms, stream);
+      return launch_one<ModeKSRk4>(f, out, rl, queue, fb, s, stream);
     case kModeBundle:
       return lam ? launch_pair<ModeBundlePair<true>>(f, out, rl, queue, fb, s, stream)
                  : launch_pair<ModeBundlePair<false>>(f, out, rl, queue, fb, s, stream);

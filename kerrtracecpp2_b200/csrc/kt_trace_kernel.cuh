@@ -219,6 +219,7 @@ static cudaError_t shape_for_pair_one(int device, LaunchShape* shape) {
   shape->block = block;
   shape->grid = sms * per_sm;
   shape->smem = smem;
+  shape->sms = sms;
   return cudaSuccess;
 }
 
@@ -237,6 +238,7 @@ static cudaError_t shape_for(int device, LaunchShape* shape) {
   shape->block = block;
   shape->grid = sms * per_sm;
   shape->smem = smem;
+  shape->sms = sms;
   return cudaSuccess;
 }
 
@@ -413,6 +415,7 @@ static cudaError_t batch_shape_pair_one(int device, LaunchShape* shape) {
   shape->block = BLOCK;
   shape->grid = sms * per_sm;
   shape->smem = smem;
+  shape->sms = sms;
   return cudaSuccess;
 }
 
@@ -441,6 +444,7 @@ static cudaError_t batch_shape_for(int device, LaunchShape* shape) {
   shape->block = BLOCK;
   shape->grid = sms * per_sm;
   shape->smem = smem;
+  shape->sms = sms;
   return cudaSuccess;
 }
 
