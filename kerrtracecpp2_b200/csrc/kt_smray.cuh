@@ -139,7 +139,8 @@ KT_HD_CALL void sm_paths(double M, const SmPrm<double>& P, const double* c, cons
       const double cs = (s == 3) ? hs : 0.5 * hs;
       for (int i = 0; i < n; ++i) u[i] = base[i] + cs * kp[i];
     }
-    sm_rhs<C>(M, P, u, c, k, &kk);
+    if constexpr (C::kInlineRhs) sm_rhs_body<C, double>(M, P, u, c, k, &kk);
+    else sm_rhs<C>(M, P, u, c, k, &kk);
     if (rec)
       for (int i = 0; i < n; ++i) {
         rec->u[t][i] = u[i];
@@ -249,7 +250,9 @@ KT_HD_CALL void sm_dp_paths(double M, const SmPrm<double>& P, const double* c, c
       const double hw = hh * dp5_a(s, j);
       for (int i = 0; i < n; ++i) u[i] = u[i] + hw * kk[j][i];
     }
-    sm_rhs<C>(M, P, u, c, kk[s], &fp);
+    double ks[n];
+    sm_rhs_body<C, double>(M, P, u, c, ks, &fp);
+    for (int i = 0; i < n; ++i) kk[s][i] = ks[i];
     if (rec)
       for (int i = 0; i < n; ++i) rec->u[s][i] = u[i];
     if (s == 6)
@@ -282,8 +285,11 @@ KT_HD int dp5_update(double err, double* h) {
     if (*h < 1e-10) *h = 1e-10;
     return -1;
   }
-  if (err <= 1.0 || *h < 1e-10) {
-    const double fac = (err > 1e-12) ? 0.9 * ktm_pow(1.0 / err, 0.2) : 4.0;
+  const bool accepted = err <= 1.0 || *h < 1e-10;
+  double p = 0.0;  // one pow for both outcomes, as in doubling_update
+  if (!accepted || err > 1e-12) p = pow_ctl(1.0 / err, accepted ? 0.2 : 0.25);
+  if (accepted) {
+    const double fac = (err > 1e-12) ? 0.9 * p : 4.0;
     double hnew = *h * fac;
     if (!finite(hnew)) hnew = *h;
     if (hnew > 100.0) hnew = 100.0;
@@ -291,7 +297,7 @@ KT_HD int dp5_update(double err, double* h) {
     *h = hnew;
     return 1;
   }
-  double hnew = (*h * 0.9) * ktm_pow(1.0 / err, 0.25);
+  double hnew = (*h * 0.9) * p;
   if (!finite(hnew)) hnew = *h * 0.5;
   *h = dmax(hnew, 1e-10);
   return 0;
@@ -597,14 +603,17 @@ KT_HD void sm_ctl_partials(double err, double tol, double h, double* dh, double*
 // evaluation at z + e1 W_k + e2 d_k (its e2 part is Hess(H) d_k, its e1 e2
 // part D^3 H[., W_k, d_k]).  A zero column cotangent skips its evaluation.
 template <class C>
+KT_HD void sm_vjp_grad(double M, const SmPrm<double>& P, const Dual<1>* y, const double* c, Dual<1>* gy,
+                       Dual<1>* gc, Dual<1>* gp) {
+  if constexpr (C::kN == 6) ChartKS::grad<Dual<1>, true, double>(M, P, y, c, gy, gc, gp);
+  else ChartBL::grad<Dual<1>, true, false, double>(M, P, y, c, gy, gc, gp);
+}
+
+template <class C>
 KT_HD_CALL void sm_vjp_f(double M, const SmPrm<double>& P, const double* u, const double* c,
                          const double* v, double* ubar, double* cbar, double* pbar) {
   if constexpr (C::kBundle) {
     sm_vjp_f<ChartBL>(M, P, u, c, v, ubar, cbar, pbar);
-    SmPrm<HDual> Ph;
-    Ph.a = HDual(P.a);
-    Ph.Q = HDual(P.Q);
-    Ph.L = HDual(P.L);
     KT_ROLLED
     for (int k = 0; k < 2; ++k) {
       const double w0 = v[4 + k], w1 = v[6 + k], w2 = v[8 + k], w3 = v[10 + k];
@@ -613,11 +622,9 @@ KT_HD_CALL void sm_vjp_f(double M, const SmPrm<double>& P, const double* u, cons
         continue;
       }
       const double dk[4] = {-w2, -w3, w0, w1};
-      HDual yh[4], ch[2], gy[4], gc[2], gp[kSmPrm];
+      HDual yh[4], gy[4], gc[2], gp[kSmPrm];
       for (int i = 0; i < 4; ++i) yh[i] = HDual(u[i], u[4 + 2 * i + k], dk[i], 0.0);
-      ch[0] = HDual(c[0]);
-      ch[1] = HDual(c[1]);
-      ChartBL::grad<HDual, true>(M, Ph, yh, ch, gy, gc, gp);
+      ChartBL::grad<HDual, true, false, double>(M, P, yh, c, gy, gc, gp);
       for (int i = 0; i < 4; ++i) {
         ubar[i] = ubar[i] + gy[i].c;
         ubar[4 + 2 * i + k] = gy[i].b;
@@ -626,19 +633,14 @@ KT_HD_CALL void sm_vjp_f(double M, const SmPrm<double>& P, const double* u, cons
       for (int q = 0; q < kSmPrm; ++q) pbar[q] = pbar[q] + gp[q].c;
     }
   } else {
-    Dual<1> yd[C::kN], cd[C::kC], gy[C::kN], gc[C::kC], gp[kSmPrm];
+    Dual<1> yd[C::kN], gy[C::kN], gc[C::kC], gp[kSmPrm];
     for (int i = 0; i < C::kX; ++i) {
       yd[i] = Dual<1>(u[i]);
       yd[i].d[0] = -v[C::kX + i];
       yd[C::kX + i] = Dual<1>(u[C::kX + i]);
       yd[C::kX + i].d[0] = v[i];
     }
-    for (int j = 0; j < C::kC; ++j) cd[j] = Dual<1>(c[j]);
-    SmPrm<Dual<1>> Pd;
-    Pd.a = Dual<1>(P.a);
-    Pd.Q = Dual<1>(P.Q);
-    Pd.L = Dual<1>(P.L);
-    C::grad(M, Pd, yd, cd, gy, gc, gp);
+    sm_vjp_grad<C>(M, P, yd, c, gy, gc, gp);
     for (int i = 0; i < C::kN; ++i) ubar[i] = gy[i].d[0];
     for (int j = 0; j < C::kC; ++j) cbar[j] = cbar[j] + gc[j].d[0];
     for (int q = 0; q < kSmPrm; ++q) pbar[q] = pbar[q] + gp[q].d[0];
