@@ -166,6 +166,8 @@ struct ModeSepRk4 {
   }
 };
 
+template <bool kLam> struct Lockstep<ModeBundlePair<kLam>> { static constexpr bool value = true; };
+
 template <> struct Defers<ModeSepRk4> { static constexpr bool value = true; };
 
 // Launch shape per mode, measured on B200 (720p config-2 frame, BL chart

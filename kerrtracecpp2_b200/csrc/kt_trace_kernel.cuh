@@ -71,6 +71,29 @@ template <class ModeT> struct Defers { static constexpr bool value = false; };
 // 128-thread blocks and refill at every idle lane by default; a mode may
 // specialise this (see kt_kernels.cu, kt_mixed.cu).
 template <class ModeT> struct Shape { static constexpr int kBlock = 128, kMinBlocks = 1, kRefill = 1; };
+// Modes whose warps go through the slots block by block, one block-wide
+// barrier per slot.  Their step loop is longer than the instruction cache
+// holds, so that free-running warps, each at its own place in it, fetch it from
+// the next level over and over; side by side they fetch it once.  Measured:
+// two-lane bundles 960 x 540 83.1 -> 76.9 ms (no-instruction stalls 1.1 per
+// issue before), mixed KS 512 x 512 7.0 -> 5.6 ms (7.2 per issue).  The other
+// kernels' loops fit, and the barriers cost them (BL DOPRI5 720p 38.0 -> 40.1,
+// KS 51.6 -> 53.9, mixed DOPRI5 14.7 -> 17.3).
+template <class ModeT> struct Lockstep { static constexpr bool value = false; };
+
+// True once the block (Lockstep) or the warp has no active ray and the queue
+// is empty for all of it; `idle`: no active ray, but rays to fetch.
+template <class ModeT>
+__device__ __forceinline__ bool all_done(bool active, bool exhausted, bool* idle) {
+  if constexpr (Lockstep<ModeT>::value) {
+    *idle = !__syncthreads_or(active);
+    return *idle && __syncthreads_and(exhausted);
+  } else {
+    *idle = !__any_sync(kFull, active);
+    return *idle && exhausted;
+  }
+}
+
 // ---- the persistent loop ---------------------------------------------------
 // One iteration of the outer loop is one adaptive attempt for every ray of
 // the warp.  At its start, idle lanes take new rays from the queue (one
@@ -113,12 +136,12 @@ __global__ void __launch_bounds__(Shape<ModeT>::kBlock, Shape<ModeT>::kMinBlocks
         }
       }
     }
-    if (!__any_sync(kFull, active)) {
-      if (exhausted) break;
-      continue;
-    }
+    bool idle;
+    if (all_done<ModeT>(active, exhausted, &idle)) break;
+    if (idle) continue;
     KT_ROLLED
     for (int s = -1; s < ModeT::kSlots; ++s) {
+      if constexpr (Lockstep<ModeT>::value) __syncthreads();
       const bool part = active && (s >= 0 || mode.needs_k1());
       if (s < 0 && !__any_sync(kFull, part)) continue;
       if (part) {
@@ -183,12 +206,12 @@ __global__ void __launch_bounds__(Shape<ModeT>::kBlock, Shape<ModeT>::kMinBlocks
       }
       __syncwarp();  // new records written by the even lanes are visible to their partners
     }
-    if (!__any_sync(kFull, active)) {
-      if (exhausted) break;
-      continue;
-    }
+    bool idle;
+    if (all_done<ModeT>(active, exhausted, &idle)) break;
+    if (idle) continue;
     KT_ROLLED
     for (int s = -1; s < ModeT::kSlots; ++s) {
+      if constexpr (Lockstep<ModeT>::value) __syncthreads();
       const bool part = active && (s >= 0 || mode.needs_k1());
       const unsigned pmask = __ballot_sync(kFull, part);
       if (s < 0 && !pmask) continue;
