@@ -90,7 +90,8 @@ struct ModeBLDopri5MixedT {
 };
 
 // KS: FP32 beyond r_fp32 unless the radial momentum x.p/|x| is small.
-template <bool kFp32>
+// kBlockwise (with kFp32): as blocks that go through the slots together.
+template <bool kFp32, bool kBlockwise = false>
 struct ModeKSRk4MixedT {
   using Machine = KSRk4;
   static constexpr int kSlots = KSRk4::kSlots;
@@ -165,12 +166,16 @@ template <bool B> struct Shape<ModeBLDopri5MixedT<B>> {
   static constexpr int kBlock = 64, kMinBlocks = KT_MIXED_DOPRI5_MINB,
                        kRefill = B ? KT_MIXED32_DOPRI5_REFILL : 32;
 };
-// KS with the FP32 branch: 256-thread blocks whose warps go through the slots
-// together (Lockstep; 512 x 512 5.6 ms, 5.8 as 320 x 2, 6.6 as 128 x 5,
-// against 7.0 free-running as 64 x 9).
-template <> struct Shape<ModeKSRk4MixedT<true>> { static constexpr int kBlock = 256, kMinBlocks = 2, kRefill = 32; };
-template <> struct Lockstep<ModeKSRk4MixedT<true>> { static constexpr bool value = true; };
-template <> struct Shape<ModeKSRk4MixedT<false>> { static constexpr int kBlock = 64, kMinBlocks = 9, kRefill = 32; };
+// KS with the FP32 branch, where the rays give every SM a block: 256-thread
+// blocks whose warps go through the slots together (Lockstep; 512 x 512 5.6 ms,
+// 5.8 as 320 x 2, 6.6 as 128 x 5, against 7.0 free-running as 64 x 9).
+// Fewer rays spread over the SMs as free-running blocks of 64 (40 x 30: 2.7 ms
+// against 2.9).  Without the branch 8 blocks of 64 (512 x 512 at tol 1e-9: 3.9 ms
+// against 4.0 with 10).
+template <> struct Shape<ModeKSRk4MixedT<true, true>> { static constexpr int kBlock = 256, kMinBlocks = 2, kRefill = 32; };
+template <> struct Lockstep<ModeKSRk4MixedT<true, true>> { static constexpr bool value = true; };
+template <> struct Shape<ModeKSRk4MixedT<true>> { static constexpr int kBlock = 64, kMinBlocks = 9, kRefill = 32; };
+template <> struct Shape<ModeKSRk4MixedT<false>> { static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32; };
 // Mixed bundles: 64-thread blocks, at least 6 per SM (168 registers, no
 // spill), measured at 1080p: 90.8 ms against 97.2 for 128 x 1 (216
 // registers), 98.3 for 128 x 3, 91.7 for 64 x 5; refilling at 16 or 8 idle
@@ -197,10 +202,12 @@ static cudaError_t launch_one(const Frame& f, const OutSoA& out, const RayList& 
   return cudaGetLastError();
 }
 
-static cudaError_t launch_ks_fp32(const Frame& f, const OutSoA& out, const RayList& rl,
-                                  uint32_t* queue, const Fallback& fb, const LaunchShape& s,
-                                  cudaStream_t stream) {
-  using M = ModeKSRk4MixedT<true>;
+// The three KS instantiations share their record and differ in block, blocks
+// per SM and so in shared memory; s is the free-running FP64 one's shape.
+template <class M>
+static cudaError_t launch_ks(const Frame& f, const OutSoA& out, const RayList& rl,
+                             uint32_t* queue, const Fallback& fb, const LaunchShape& s,
+                             cudaStream_t stream) {
   LaunchShape t = s;
   t.block = Shape<M>::kBlock;
   t.grid = s.sms * Shape<M>::kMinBlocks;
@@ -215,9 +222,9 @@ cudaError_t launch_shape_mixed(Mode mode, int device, LaunchShape* shape) {
     case kModeBLRk4Mixed: return shape_for<ModeBLRk4MixedT<true>>(device, shape);
     case kModeBLDopri5Mixed: return shape_for<ModeBLDopri5MixedT<true>>(device, shape);
     case kModeKSRk4Mixed: {
-      // the FP32 instantiation has a shape of its own (launch_ks_fp32); its
-      // shared memory is set up here
-      const cudaError_t e = shape_for<ModeKSRk4MixedT<true>>(device, shape);
+      // the other instantiations' shared memory is set up here (launch_ks)
+      cudaError_t e = shape_for<ModeKSRk4MixedT<true, true>>(device, shape);
+      if (e == cudaSuccess) e = shape_for<ModeKSRk4MixedT<true>>(device, shape);
       return e != cudaSuccess ? e : shape_for<ModeKSRk4MixedT<false>>(device, shape);
     }
     case kModeBundleMixed: return shape_for<ModeBundleMixed>(device, shape);
@@ -237,8 +244,10 @@ cudaError_t launch_trace_mixed(Mode mode, const Frame& f, const OutSoA& out, con
       return fp32 ? launch_one<ModeBLDopri5MixedT<true>>(f, out, rl, queue, fb, s, stream)
                   : launch_one<ModeBLDopri5MixedT<false>>(f, out, rl, queue, fb, s, stream);
     case kModeKSRk4Mixed:
-      return fp32 ? launch_ks_fp32(f, out, rl, queue, fb, s, stream)
-                  : launch_one<ModeKSRk4MixedT<false>>(f, out, rl, queue, fb, s, stream);
+      if (!fp32) return launch_one<ModeKSRk4MixedT<false>>(f, out, rl, queue, fb, s, stream);
+      return !rl.n_dev && rl.n < (uint32_t)(256 * s.sms)
+                 ? launch_ks<ModeKSRk4MixedT<true>>(f, out, rl, queue, fb, s, stream)
+                 : launch_ks<ModeKSRk4MixedT<true, true>>(f, out, rl, queue, fb, s, stream);
     case kModeBundleMixed: return launch_one<ModeBundleMixed>(f, out, rl, queue, fb, s, stream);
     default: return cudaErrorInvalidValue;
   }
