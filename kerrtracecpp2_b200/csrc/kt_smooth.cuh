@@ -110,13 +110,11 @@ struct ChartKS {
   static constexpr bool kInlineRhs = false;  // sm_paths' form of the RHS
 
   // gy = dH/dy (X, Y, Z, pX, pY, pZ), gc = dH/dp_T, gp = dH/d(a, Q, Lambda)
-  // (only with kPrm: the right-hand side needs gy and gc alone).  PT: the type
-  // of the parameters and constants, double where only y carries tangents.
-  template <class T, bool kPrm = true, class PT = T>
-  KT_HD static void grad(double M, const SmPrm<PT>& P, const T* y, const PT* c, T* gy, T* gc, T* gp) {
-    const T &X = y[0], &Y = y[1], &Z = y[2], &pX = y[3], &pY = y[4], &pZ = y[5];
-    const PT& pT = c[0];
-    const PT a = P.a, a2 = P.a * P.a;
+  // (only with kPrm: the right-hand side needs gy and gc alone).
+  template <class T, bool kPrm = true>
+  KT_HD static void grad(double M, const SmPrm<T>& P, const T* y, const T* c, T* gy, T* gc, T* gp) {
+    const T &X = y[0], &Y = y[1], &Z = y[2], &pX = y[3], &pY = y[4], &pZ = y[5], &pT = c[0];
+    const T a = P.a, a2 = P.a * P.a;
     const T R2 = X * X + Y * Y + Z * Z;
     const T b = R2 - a2;
     const T r = sm_sqrt(0.5 * (b + sm_sqrt(b * b + 4.0 * a2 * Z * Z)));
@@ -622,10 +620,13 @@ KT_HD double sm_hermite_da(double y0, double y1, double d0, double d1, double h,
 
 // First crossing of `target` in [0, 1] (first_event_alpha_hermite,
 // geodesic.hpp:104-140: 8 bins scanned in order) refined to convergence:
-// bisection while the bracket is wide, then safeguarded Newton steps.
+// bisection while the bracket is wide, then safeguarded Newton steps.  kQuick:
+// no_event first (the BL kernels; the KS one, larger than the instruction
+// cache already, measured slower with it).
+template <bool kQuick>
 KT_HD bool sm_first_crossing(double y0, double y1, double d0, double d1, double h, double target,
                              double* alpha) {
-  if (no_event(y0, y1, d0, d1, h, target)) return false;
+  if (kQuick && no_event(y0, y1, d0, d1, h, target)) return false;
   const double f_eps = 1e-12;
   double a0 = 0.0, f0 = y0 - target;
   if (fabs(f0) <= f_eps) {
