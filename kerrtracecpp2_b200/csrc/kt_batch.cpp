@@ -71,6 +71,11 @@ int default_refill(kt::Mode m) {
   return m == kt::kModeBundle ? 8 : m == kt::kModeSepRk4 ? 1 : 32;
 }
 
+// Whether a group's frames are interleaved (launch_batch_order).  Not with the
+// mixed tracer's FP32 branch, which a warp takes or not by all its 32 rays: in
+// sequence the warps' rays are those they have always been.
+bool interleaved(const Group& g) { return g.frames.size() > 1 && !g.fp32; }
+
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
@@ -354,8 +359,16 @@ kt_status kt_batch_create(kt_context* ctx, const kt_frame_desc* descs, const kt_
   bytes = align256(bytes + counters_bytes);
   const size_t off_scratch = bytes;
   bytes = align256(bytes + ring_scratch * sizeof(uint32_t));
+  // the largest interleaved group's rays, frame after frame (in the batch's one
+  // allocation: an allocation and a free of its own cost the set-up 1 ms)
+  uint64_t n_largest = 0;
+  for (const Group& g : b->groups)
+    if (interleaved(g)) n_largest = std::max(n_largest, g.n_rays);
+  const size_t off_seq = bytes;
+  bytes = align256(bytes + n_largest * sizeof(uint32_t));
   KT_CUDA(ctx, cudaMalloc((void**)&b->d_mem, bytes), "batch buffers");
   uint32_t* d_counters = (uint32_t*)(b->d_mem + off_counters);
+  uint32_t* d_seq = (uint32_t*)(b->d_mem + off_seq);
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
     Group& g = b->groups[gi];
     const size_t nf = g.frames.size();
@@ -383,9 +396,13 @@ kt_status kt_batch_create(kt_context* ctx, const kt_frame_desc* descs, const kt_
     for (size_t k = 0; k < nf; ++k) {
       const kt_frame_desc& dk = descs[g.frames[k]];
       KT_CUDA(ctx, kt::launch_ring_order(dk.width, dk.height, (uint32_t)hoff[k],
-                                         (uint32_t*)(b->d_mem + off_scratch), g.d_order + hoff[k],
+                                         (uint32_t*)(b->d_mem + off_scratch),
+                                         (interleaved(g) ? d_seq : g.d_order) + hoff[k],
                                          ctx->stream), "ray order");
     }
+    if (interleaved(g))
+      KT_CUDA(ctx, kt::launch_batch_order(g.d_offsets, (int)nf, g.n_rays, d_seq, g.d_order, ctx->stream),
+              "ray order");
     KT_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "ray order");
     if (kt::has_fallback(g.mode)) {
       g.fb_variant = default_variant(g.fb_mode);
@@ -407,7 +424,7 @@ kt_status kt_batch_create(kt_context* ctx, const kt_frame_desc* descs, const kt_
     in.n_rays = g.n_rays;
     in.variant = g.variant;
     in.block = kt::kBatchBlock[g.variant];
-    in.min_blocks = kt::kBatchMinBlocks[g.variant];
+    in.min_blocks = kt::batch_min_blocks(g.mode, g.variant);
     in.grid = g.shape.grid;
     in.refill_min = g.refill_min;
     in.rays_per_warp = kt::kBatchRaysPerWarp[g.variant];

@@ -152,6 +152,12 @@ struct BatchRays {
 constexpr int kBatchVariants = 4;
 constexpr int kBatchBlock[kBatchVariants] = {64, 128, 64, 128};
 constexpr int kBatchMinBlocks[kBatchVariants] = {9, 1, 12, 3};
+// The exact BL and KS kernels take 8 blocks for variant 0, as their
+// single-frame kernels do (128 registers; at 64 x 9 they spill: a batch of 12
+// frames of 256 x 256, in sequence, 44.0 ms, 41.6 with 8).
+constexpr int batch_min_blocks(Mode m, int v) {
+  return v == 0 && (m == kModeBLRk4 || m == kModeBLDopri5 || m == kModeKSRk4) ? 8 : kBatchMinBlocks[v];
+}
 // Variant 3 runs two lanes per ray (16 rays per warp); only the FP64 bundle
 // kernel has that form.
 constexpr int kBatchPairVariant = 3;
@@ -168,6 +174,17 @@ cudaError_t launch_batch(Mode mode, int variant, const BatchRays& br, uint32_t* 
 cudaError_t batch_shape_mixed(Mode mode, int variant, int device, LaunchShape* shape);
 cudaError_t launch_batch_mixed(Mode mode, int variant, const BatchRays& br, uint32_t* queue,
                                const Fallback& fb, const LaunchShape& s, cudaStream_t st);
+
+// The order of a batch group's rays: `in` lists each frame's rays in its own
+// order, one frame after another; `out` the same rays, in chunks of 32 of one
+// frame, the frames' chunks interleaved in proportion: chunk j of a frame
+// with F chunks goes by (j + 1/2) / F.  Every frame's long rays (first in its
+// centre-out order) then start early, where the frames in sequence left the
+// last one's for the end of the launch (12 Kerr frames of 256 x 256 41.6 ms,
+// 37.2 interleaved).  The rays beyond a frame's last whole chunk come at the
+// end.  offsets: the frames' first rays (n_frames + 1).
+cudaError_t launch_batch_order(const uint64_t* offsets, int n_frames, uint64_t n_rays,
+                               const uint32_t* in, uint32_t* out, cudaStream_t stream);
 
 // Centre-out ray order (kt_kernels.cu): base + the W x H frame's pixels in
 // rings about the image centre, innermost first, in blocks of 8 x 4 pixels

@@ -187,6 +187,10 @@ template <> struct Defers<ModeSepRk4> { static constexpr bool value = true; };
 template <class M, bool kLam> struct Shape<ModeBL<M, kLam>> {
   static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32;
 };
+template <class M, bool kLam> struct BatchMin0<ModeBL<M, kLam>> {
+  static constexpr int value = batch_min_blocks(kModeBLRk4, 0);
+};
+template <> struct BatchMin0<ModeKSRk4> { static constexpr int value = batch_min_blocks(kModeKSRk4, 0); };
 // (720p KS frame 51.6 ms against 52.3 with 10 blocks of 96 registers.)
 template <> struct Shape<struct ModeKSRk4> { static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32; };
 template <> struct Shape<struct ModeBundle> { static constexpr int kBlock = 128, kMinBlocks = 1, kRefill = 16; };
@@ -466,6 +470,60 @@ cudaError_t launch_ring_order(int W, int H, uint32_t base, uint32_t* scratch, ui
   k_ring_count<<<tiles, 256, 0, stream>>>(W, H, tile, tiles, scratch);
   k_ring_scan<<<1, 1024, 0, stream>>>(scratch, (uint32_t)kOrderClasses * tiles);
   k_ring_place<<<tiles, 32, 0, stream>>>(W, H, tile, tiles, scratch, base, list);
+  return cudaGetLastError();
+}
+
+// ---- the order of a batch ----------------------------------------------------
+
+// #{i in [0, F_m) : (i + 1/2) / F_m < (j + 1/2) / F_k, or equal and m < k}
+// = the odd t with t F_k < N (or <= N), N = (2 j + 1) F_m.
+__device__ __forceinline__ uint64_t chunks_before(uint64_t N, uint64_t D, bool equal_counts) {
+  uint64_t c = ((N - 1) / D + 1) / 2;
+  if (equal_counts && N % D == 0 && ((N / D) & 1u)) ++c;
+  return c;
+}
+
+// One warp per chunk of 32 rays; the warps past the last chunk copy the rays
+// beyond each frame's whole chunks.
+__global__ void k_batch_order(const uint64_t* __restrict__ offsets, int nf,
+                              const uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint64_t n = offsets[nf];
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  uint64_t whole = 0;
+  for (int m = 0; m < nf; ++m) whole += (offsets[m + 1] - offsets[m]) / 32;
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < whole + (uint64_t)nf; w += warps) {
+    if (w < whole) {  // chunk j of frame k
+      int k = 0;
+      uint64_t j = w;
+      for (;; ++k) {
+        const uint64_t F = (offsets[k + 1] - offsets[k]) / 32;
+        if (j < F) break;
+        j -= F;
+      }
+      const uint64_t Fk = (offsets[k + 1] - offsets[k]) / 32;
+      uint64_t rank = 0;
+      for (int m = 0; m < nf; ++m) {
+        const uint64_t Fm = (offsets[m + 1] - offsets[m]) / 32;
+        if (Fm) rank += chunks_before((2 * j + 1) * Fm, Fk, m < k);
+      }
+      out[rank * 32 + lane] = in[offsets[k] + j * 32 + lane];
+    } else {  // frame k's remainder
+      const int k = (int)(w - whole);
+      uint64_t at = whole * 32;
+      for (int m = 0; m < k; ++m) at += (offsets[m + 1] - offsets[m]) % 32;
+      const uint64_t first = offsets[k + 1] - (offsets[k + 1] - offsets[k]) % 32;
+      if (first + lane < offsets[k + 1] && at + lane < n) out[at + lane] = in[first + lane];
+    }
+  }
+}
+
+cudaError_t launch_batch_order(const uint64_t* offsets, int n_frames, uint64_t n_rays,
+                               const uint32_t* in, uint32_t* out, cudaStream_t stream) {
+  const uint64_t warps = n_rays / 32 + (uint64_t)n_frames;
+  uint64_t grid = (warps + 7) / 8;
+  if (grid > 148 * 8) grid = 148 * 8;
+  k_batch_order<<<(int)grid, 256, 0, stream>>>(offsets, n_frames, in, out);
   return cudaGetLastError();
 }
 

@@ -471,11 +471,14 @@ static cudaError_t batch_shape_for(int device, LaunchShape* shape) {
   return cudaSuccess;
 }
 
+// Minimum blocks of variant 0 (batch_min_blocks, kt_internal.h).
+template <class ModeT> struct BatchMin0 { static constexpr int value = kBatchMinBlocks[0]; };
+
 // One case per entry of kBatchBlock / kBatchMinBlocks (kt_internal.h).
 template <class ModeT>
 static cudaError_t batch_shape(int variant, int device, LaunchShape* s) {
   switch (variant) {
-    case 0: return batch_shape_for<ModeT, 64, 9>(device, s);
+    case 0: return batch_shape_for<ModeT, 64, BatchMin0<ModeT>::value>(device, s);
     case 1: return batch_shape_for<ModeT, 128, 1>(device, s);
     case 2: return batch_shape_for<ModeT, 64, 12>(device, s);
   }
@@ -496,7 +499,7 @@ template <class ModeT>
 static cudaError_t batch_launch(int variant, const BatchRays& br, uint32_t* queue,
                                 const Fallback& fb, const LaunchShape& s, cudaStream_t st) {
   switch (variant) {
-    case 0: k_trace_batch<ModeT, 64, 9><<<s.grid, s.block, s.smem, st>>>(br, queue, fb); break;
+    case 0: k_trace_batch<ModeT, 64, BatchMin0<ModeT>::value><<<s.grid, s.block, s.smem, st>>>(br, queue, fb); break;
     case 1: k_trace_batch<ModeT, 128, 1><<<s.grid, s.block, s.smem, st>>>(br, queue, fb); break;
     case 2: k_trace_batch<ModeT, 64, 12><<<s.grid, s.block, s.smem, st>>>(br, queue, fb); break;
     default: return cudaErrorInvalidValue;
