@@ -30,7 +30,8 @@ NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "--fmad=false", "-lineinfo", "-Xptxas"
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall", "-Wextra",
              "-I", os.path.join(CUDA_HOME, "include")]
 
-CU_SOURCES = ["kt_kernels.cu", "kt_noalloc.cu", "kt_mixed.cu", "kt_adjoint.cu"]
+CU_SOURCES = ["kt_kernels.cu", "kt_noalloc.cu", "kt_mixed.cu",
+              "kt_mixed_bundle.cu", "kt_adjoint.cu"]
 CXX_SOURCES = ["kt_frame.cpp", "kt_api.cpp", "kt_batch.cpp", "kt_grad.cpp", "kt_io.cpp",
                "kt_compat.cpp"]
 HEADERS = ["ktmath.h", "kt_exact.cuh", "kt_group.cuh", "ktmath_consts.h", "kt_physics.cuh", "kt_machines.cuh", "kt_internal.h",
@@ -39,7 +40,7 @@ HEADERS = ["ktmath.h", "kt_exact.cuh", "kt_group.cuh", "ktmath_consts.h", "kt_ph
 # Per-file compile flags: the exact kernels keep every multiply and add of
 # the reference's arithmetic separate; the mixed-precision kernels are not
 # compared bit for bit and use FMA contraction.
-CU_FLAGS = {"kt_mixed.cu": ["--fmad=true"]}
+CU_FLAGS = {"kt_mixed.cu": ["--fmad=true"], "kt_mixed_bundle.cu": ["--fmad=true"]}
 # The frame set-up evaluates the independent samples of the horizon scan and
 # the ISCO search on several host threads.
 CXX_FILE_FLAGS = {"kt_frame.cpp": ["-fopenmp"]}

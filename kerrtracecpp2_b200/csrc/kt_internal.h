@@ -120,6 +120,11 @@ cudaError_t launch_shape_mixed(Mode mode, int device, LaunchShape* shape);
 cudaError_t launch_trace_mixed(Mode mode, const Frame& f, const OutSoA& out, const RayList& rl,
                                uint32_t* queue, const Fallback& fb, const LaunchShape& shape,
                                cudaStream_t stream);
+// Their bundle kernel (kt_mixed_bundle.cu).
+cudaError_t launch_shape_mixed_bundle(int device, LaunchShape* shape);
+cudaError_t launch_trace_mixed_bundle(const Frame& f, const OutSoA& out, const RayList& rl,
+                                      uint32_t* queue, const Fallback& fb, const LaunchShape& s,
+                                      cudaStream_t stream);
 
 // ---- batches of frames (k_trace_batch, kt_trace_kernel.cuh) ---------------
 // Ray g of a batch is pixel g - offsets[k] of frame k, where offsets[k] <= g
@@ -174,6 +179,9 @@ cudaError_t launch_batch(Mode mode, int variant, const BatchRays& br, uint32_t* 
 cudaError_t batch_shape_mixed(Mode mode, int variant, int device, LaunchShape* shape);
 cudaError_t launch_batch_mixed(Mode mode, int variant, const BatchRays& br, uint32_t* queue,
                                const Fallback& fb, const LaunchShape& s, cudaStream_t st);
+cudaError_t batch_shape_mixed_bundle(int variant, int device, LaunchShape* shape);
+cudaError_t launch_batch_mixed_bundle(int variant, const BatchRays& br, uint32_t* queue,
+                                      const Fallback& fb, const LaunchShape& s, cudaStream_t st);
 
 // The order of a batch group's rays: `in` lists each frame's rays in its own
 // order, one frame after another; `out` the same rays, in chunks of 32 of one

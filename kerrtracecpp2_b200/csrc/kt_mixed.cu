@@ -1,4 +1,5 @@
-// kt_mixed.cu -- mixed-precision trace kernels (KT_PREC_MIXED).
+// kt_mixed.cu -- mixed-precision trace kernels (KT_PREC_MIXED); the bundle one is
+// in kt_mixed_bundle.cu.
 //
 // Same persistent loop and the same FP64 integrators as the exact kernels
 // (state, stage sums, embedded error estimate, step-size controller, event
@@ -15,7 +16,6 @@
 // are compared with the FP64 oracle statistically.
 #include <cmath>
 
-#include "kt_smooth.cuh"
 #include "kt_trace_kernel.cuh"
 
 namespace kt {
@@ -127,23 +127,6 @@ struct ModeKSRk4MixedT {
   }
 };
 
-struct ModeBundleMixed {
-  using Machine = Bundle;
-  static constexpr int kSlots = Bundle::kSlots;
-  Bundle* m;
-  __device__ __forceinline__ bool needs_k1() const { return m->needs_k1(); }
-  __device__ __forceinline__ bool start(const Frame& f, uint32_t pix, uint32_t, uint32_t, const Fallback&) {
-    m->init(f, (int)(pix % (uint32_t)f.cam.W), (int)(pix / (uint32_t)f.cam.W));
-    return true;
-  }
-  __device__ __forceinline__ bool slot(const Frame& f, int s, RayResult* res) {
-    double y[4], yW[8], k[5], kW[8];
-    m->input(s, y, yW);
-    bundle_rhs_analytic(f.g, y, m->pt, m->pphi, yW, k, kW);
-    return m->consume(f, s, k, kW, res);
-  }
-};
-
 // Launch shapes, measured on B200 as for the exact kernels: refilling a
 // warp only when all 32 lanes are idle matters more here, since the FP32/FP64
 // choice is made per warp and a warp of neighbouring rays that started
@@ -176,24 +159,6 @@ template <> struct Shape<ModeKSRk4MixedT<true, true>> { static constexpr int kBl
 template <> struct Lockstep<ModeKSRk4MixedT<true, true>> { static constexpr bool value = true; };
 template <> struct Shape<ModeKSRk4MixedT<true>> { static constexpr int kBlock = 64, kMinBlocks = 9, kRefill = 32; };
 template <> struct Shape<ModeKSRk4MixedT<false>> { static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32; };
-// Mixed bundles: 64-thread blocks, at least 6 per SM (168 registers, no
-// spill), measured at 1080p: 90.8 ms against 97.2 for 128 x 1 (216
-// registers), 98.3 for 128 x 3, 91.7 for 64 x 5; refilling at 16 or 8 idle
-// lanes 101.0 / 101.6.
-#ifndef KT_MIXED_BUNDLE_BLOCK
-#define KT_MIXED_BUNDLE_BLOCK 64
-#endif
-#ifndef KT_MIXED_BUNDLE_MINB
-#define KT_MIXED_BUNDLE_MINB 6
-#endif
-#ifndef KT_MIXED_BUNDLE_REFILL
-#define KT_MIXED_BUNDLE_REFILL 32
-#endif
-template <> struct Shape<ModeBundleMixed> {
-  static constexpr int kBlock = KT_MIXED_BUNDLE_BLOCK, kMinBlocks = KT_MIXED_BUNDLE_MINB,
-                       kRefill = KT_MIXED_BUNDLE_REFILL;
-};
-
 template <class ModeT>
 static cudaError_t launch_one(const Frame& f, const OutSoA& out, const RayList& rl,
                               uint32_t* queue, const Fallback& fb, const LaunchShape& s,
@@ -227,7 +192,7 @@ cudaError_t launch_shape_mixed(Mode mode, int device, LaunchShape* shape) {
       if (e == cudaSuccess) e = shape_for<ModeKSRk4MixedT<true>>(device, shape);
       return e != cudaSuccess ? e : shape_for<ModeKSRk4MixedT<false>>(device, shape);
     }
-    case kModeBundleMixed: return shape_for<ModeBundleMixed>(device, shape);
+    case kModeBundleMixed: return launch_shape_mixed_bundle(device, shape);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -248,7 +213,7 @@ cudaError_t launch_trace_mixed(Mode mode, const Frame& f, const OutSoA& out, con
       return !rl.n_dev && rl.n < (uint32_t)(256 * s.sms)
                  ? launch_ks<ModeKSRk4MixedT<true>>(f, out, rl, queue, fb, s, stream)
                  : launch_ks<ModeKSRk4MixedT<true, true>>(f, out, rl, queue, fb, s, stream);
-    case kModeBundleMixed: return launch_one<ModeBundleMixed>(f, out, rl, queue, fb, s, stream);
+    case kModeBundleMixed: return launch_trace_mixed_bundle(f, out, rl, queue, fb, s, stream);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -258,7 +223,7 @@ cudaError_t batch_shape_mixed(Mode mode, int variant, int device, LaunchShape* s
     case kModeBLRk4Mixed: return batch_shape<ModeBLRk4MixedT<true>>(variant, device, shape);
     case kModeBLDopri5Mixed: return batch_shape<ModeBLDopri5MixedT<true>>(variant, device, shape);
     case kModeKSRk4Mixed: return batch_shape<ModeKSRk4MixedT<true>>(variant, device, shape);
-    case kModeBundleMixed: return batch_shape<ModeBundleMixed>(variant, device, shape);
+    case kModeBundleMixed: return batch_shape_mixed_bundle(variant, device, shape);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -275,7 +240,7 @@ cudaError_t launch_batch_mixed(Mode mode, int variant, const BatchRays& br, uint
     case kModeKSRk4Mixed:
       return br.fp32 ? batch_launch<ModeKSRk4MixedT<true>>(variant, br, queue, fb, s, st)
                      : batch_launch<ModeKSRk4MixedT<false>>(variant, br, queue, fb, s, st);
-    case kModeBundleMixed: return batch_launch<ModeBundleMixed>(variant, br, queue, fb, s, st);
+    case kModeBundleMixed: return launch_batch_mixed_bundle(variant, br, queue, fb, s, st);
     default: return cudaErrorInvalidValue;
   }
 }

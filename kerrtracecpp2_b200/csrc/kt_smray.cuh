@@ -615,7 +615,7 @@ KT_HD void sm_vjp_grad(double M, const SmPrm<double>& P, const Dual<1>* y, const
     const Dual<1> cd[1] = {Dual<1>(c[0])};
     ChartKS::grad<Dual<1>>(M, Pd, y, cd, gy, gc, gp);
   } else {
-    ChartBL::grad<Dual<1>, true, false, double>(M, P, y, c, gy, gc, gp);
+    ChartBL::grad<Dual<1>, true, double>(M, P, y, c, gy, gc, gp);
   }
 }
 
@@ -634,7 +634,7 @@ KT_HD_CALL void sm_vjp_f(double M, const SmPrm<double>& P, const double* u, cons
       const double dk[4] = {-w2, -w3, w0, w1};
       HDual yh[4], gy[4], gc[2], gp[kSmPrm];
       for (int i = 0; i < 4; ++i) yh[i] = HDual(u[i], u[4 + 2 * i + k], dk[i], 0.0);
-      ChartBL::grad<HDual, true, false, double>(M, P, yh, c, gy, gc, gp);
+      ChartBL::grad<HDual, true, double>(M, P, yh, c, gy, gc, gp);
       for (int i = 0; i < 4; ++i) {
         ubar[i] = ubar[i] + gy[i].c;
         ubar[4 + 2 * i + k] = gy[i].b;

@@ -237,8 +237,12 @@ static __host__ __device__ __noinline__ void ktm_sincos_rest(double x, double* s
 #define ktm_sincos_rest ktm_sincos_any
 #endif
 KTM_FN void ktm_sincos(double x, double* s, double* c) {
+#if defined(__CUDA_ARCH__) && defined(KTM_SINCOS_CASES)
+  ktm_sincos_any(x, s, c);
+#else
   if (ktm_sincos_plain(x)) ktm_sincos_core(x, s, c);
   else ktm_sincos_rest(x, s, c);
+#endif
 }
 
 KTM_FN double ktm_sin(double x) {
