@@ -27,7 +27,7 @@
 
 namespace kt {
 
-constexpr int kSmBlock = 64;
+constexpr int kSmBlock = 64, kSmWide = 256;
 constexpr int kSumBlocks = 296;
 constexpr int kSumThreads = 256;
 
@@ -38,8 +38,15 @@ constexpr int kSumThreads = 256;
 // blocks the 320x180 bundle gradient takes 85 / 85 / 100 ms against 71, to 5
 // blocks the 512x512 KS one 44 against 33 and the 640x360 DOPRI5 one 42
 // against 30: the spills cost more than the warps bring.
-template <class C, bool kGrad, class I>
-__global__ void __launch_bounds__(kSmBlock) k_smooth(const Frame f, const OutSoA out, const SmJob job,
+// kBlock = kSmWide: the block's 256 rays are taken together, so that its warps
+// start a ray, and near enough its reverse sweep, side by side: these kernels
+// wait for instructions (their loops are larger than the instruction cache;
+// half the warps per SM are as fast), and a warp that follows another finds
+// them fetched.  640x360 DOPRI5 26.7 -> 23.5 ms, 320x180 bundles 68.9 ->
+// 66.0; groups of 64 or 128 gained nothing.  Fewer rays than 256 per SM leave
+// SMs without a block and keep the 64-thread ones.
+template <class C, bool kGrad, class I, int kBlock>
+__global__ void __launch_bounds__(kBlock) k_smooth(const Frame f, const OutSoA out, const SmJob job,
                                                      uint32_t n, const uint32_t* __restrict__ list,
                                                      uint32_t n_list,
                                                      const uint32_t* __restrict__ n_dev,
@@ -51,11 +58,20 @@ __global__ void __launch_bounds__(kSmBlock) k_smooth(const Frame f, const OutSoA
   const unsigned lane = threadIdx.x & 31u;
   KT_ROLLED
   for (;;) {
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(queue, 32u);
-    base = __shfl_sync(kFull, base, 0);
+    uint32_t base = 0, i;
+    if constexpr (kBlock == kSmWide) {
+      __shared__ uint32_t first;
+      __syncthreads();
+      if (threadIdx.x == 0) first = atomicAdd(queue, (uint32_t)kBlock);
+      __syncthreads();
+      base = first;
+      i = base + threadIdx.x;
+    } else {
+      if (lane == 0) base = atomicAdd(queue, 32u);
+      base = __shfl_sync(kFull, base, 0);
+      i = base + lane;
+    }
     if (base >= count) break;
-    const uint32_t i = base + lane;
     const uint32_t pix = i < count ? (list ? list[i] : i) : n;
     if (pix < n) {  // else past the end, or a caller's list index outside the frame
       RayResult o;
@@ -162,20 +178,34 @@ static cudaError_t tangent_launch(const Frame& f, const OutSoA& out, uint32_t n,
   return cudaGetLastError();
 }
 
+template <class C, bool kGrad, class I, int kBlock>
+static cudaError_t smooth_launch_as(const Frame& f, const OutSoA& out, uint32_t n, const SmJob& job,
+                                    const uint32_t* list, uint32_t n_list, const uint32_t* n_dev,
+                                    uint32_t* queue, uint32_t* fb_pix, uint32_t* fb_n, int sms,
+                                    cudaStream_t st) {
+  int per_sm = 0;
+  const cudaError_t e =
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_smooth<C, kGrad, I, kBlock>, kBlock, 0);
+  if (e != cudaSuccess) return e;
+  const int grid = sms * (per_sm < 1 ? 1 : per_sm);
+  k_smooth<C, kGrad, I, kBlock><<<grid, kBlock, 0, st>>>(f, out, job, n, list, n_list, n_dev, queue,
+                                                         fb_pix, fb_n);
+  return cudaGetLastError();
+}
+
 template <class C, bool kGrad, class I = SmRk4>
 static cudaError_t smooth_launch(const Frame& f, const OutSoA& out, uint32_t n, const SmJob& job,
                                  const uint32_t* list, uint32_t n_list, const uint32_t* n_dev,
                                  uint32_t* queue,
                                  uint32_t* fb_pix, uint32_t* fb_n, int device, cudaStream_t st) {
-  int sms = 0, per_sm = 0;
-  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  int sms = 0;
+  const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_smooth<C, kGrad, I>, kSmBlock, 0);
-  if (e != cudaSuccess) return e;
-  const int grid = sms * (per_sm < 1 ? 1 : per_sm);
-  k_smooth<C, kGrad, I><<<grid, kSmBlock, 0, st>>>(f, out, job, n, list, n_list, n_dev, queue, fb_pix,
-                                                    fb_n);
-  return cudaGetLastError();
+  if (kGrad && !n_dev && (list ? n_list : n) >= (uint32_t)kSmWide * (uint32_t)sms)
+    return smooth_launch_as<C, kGrad, I, kGrad ? kSmWide : kSmBlock>(f, out, n, job, list, n_list, n_dev,
+                                                                     queue, fb_pix, fb_n, sms, st);
+  return smooth_launch_as<C, kGrad, I, kSmBlock>(f, out, n, job, list, n_list, n_dev, queue, fb_pix, fb_n,
+                                                 sms, st);
 }
 
 cudaError_t launch_smooth(const Frame& f, const OutSoA& out, uint32_t n, const SmJob* job,
