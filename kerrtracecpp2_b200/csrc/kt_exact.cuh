@@ -69,7 +69,8 @@ KT_EX uint32_t top_ones(double b) {
   return (h + 4u) ^ h;
 }
 
-// 1/b within 2^-19.  The host twin of the hardware seed keeps 20 bits.
+// 1/b within 2^-19 (the hardware's largest error, over every significand, is
+// 2^-19.94; tests/exact_device.cu).  The host twin keeps 20 bits.
 KT_EX double rcp_seed(double b) {
 #if defined(__CUDA_ARCH__)
   double y;
@@ -84,14 +85,14 @@ KT_EX double rcp_seed(double b) {
 struct Rcp {
   double b, y1, y2;
 };
-KT_EX Rcp make_rcp(double b) {
+KT_EX Rcp make_rcp_seeded(double b, double y0) {
   Rcp R;
   R.b = b;
-  const double y0 = rcp_seed(b);
   R.y1 = fma(fma(-b, y0, 1.0), y0, y0);
   R.y2 = fma(fma(-b, R.y1, 1.0), R.y1, R.y1);
   return R;
 }
+KT_EX Rcp make_rcp(double b) { return make_rcp_seeded(b, rcp_seed(b)); }
 // RN(a / b); a zero numerator gives a zero of either sign (quot_signed: of
 // the quotient's).
 KT_EX double quot(double a, const Rcp& R) {
@@ -116,19 +117,28 @@ KT_EX Rcp make_rcp_from(double b, double y1) {
 // RN(sqrt(x)), and 1/sqrt(x) within 2^-52, which the quotients by the root
 // and by its square start from (make_rcp_from).  Markstein's correction
 // g + (x - g^2) h of an approximate root g, h = 1/(2 sqrt(x)):
-//   y0 = 1/sqrt(x) within 2^-19 (the hardware seed); e = 1 - x y0^2, whose
-//   rounding of x y0 leaves an error of 2^-53; y = y0 (1 + e/2 + 3 e^2/8),
-//   within 1.6 x 2^-53 of 1/sqrt(x) (series 2^-58, e 2^-54, rounding 2^-53);
+//   y0 = 1/sqrt(x) within 2^-19 (the hardware seed: 2^-20.03);
+//   e = 1 - RN(x y0) y0, y = y0 (1 + e/2 + 3 e^2/8) = (1 + d)/sqrt(x);
 //   g = RN(x y), then two corrections with h = y/2.
-// The first leaves g within (1/2 + 2^-40) ulp.  For the second write, with
-// u = ulp(g) and x scaled into [1, 4), g = K u and x - g^2 = D u^2 (exact in
-// the fma): sqrt(x) < g + u/2 means D <= K, and the result stays at g when
-// |D| (1 + d) < K, d = 2 g h - 1, |d| <= 1.6 x 2^-53.  x is a multiple of
-// 2^52 u^2, so K^2 + D is one of 2^52; with D = +-(K - j) or +-(K + j) that
-// makes j even, and j = 0 only for K = 2^52 and K = 2^53 - 1, that is x next
-// to a power of four, which the range test hands to sqrt().  From j >= 2
-// on, |D| and K differ by 2/K >= 2^-52 > |d|, so the comparison is decided
-// as the exact root decides it.
+// Scale x into [1, 4) and write sqrt(x) = K u with u = 2^-52, 2^52 <= K < 2^53,
+// k = K/2^53.  In units of 2^-53, d has
+//   1/(4 k) from the rounding of x y0 < 2 (half an ulp, 2^-53, over sqrt(x) =
+//     2 k, halved by e/2; x y0 < 2 because x < 4 (1 - 2^-18), below),
+//   0.157 from the term 5 e^3/16 left out, |e| < 2^-18 (1 + 2^-20),
+//   k from y's own rounding (half an ulp of a number below 1), and less than
+//   2^-15 from e's, the polynomial's and the product's:
+// |d| k 2^53 < 1/4 + 0.157 k + k^2 + 2^-15 < 1.41, that is |d| < 1.41/K.
+// The first correction leaves g within (1/2 + 2^-40) ulp.  For the second let
+// g = K u now be its result and x - g^2 = D u^2 (exact in the fma: |D| < K +
+// 2^14 < 2^53), so that sqrt(x) is g + D/(2 K) (1 - D/(4 K^2)) ulp and the
+// correction adds c = D/(2 K) (1 - D/(2 K^2)) (1 + d) ulp, up to K^-2.
+// RN(sqrt(x)) is g exactly when -K < D <= K, and the result is g when
+// |c| < 1/2.  x is a multiple of 2^52 u^2, so K^2 + D is one of 2^52; with
+// |D| = K + j (j of either sign) that makes j even, and j = 0 only for K = 2^52
+// and K = 2^53 - 1, that is x next to a power of four, which the range test
+// hands to sqrt().  From |j| >= 2 on, 2 |c| = (1 + j/K)(1 -+ 1/(2 K))(1 + d)
+// lies on the side of 1 that j's sign says when |d| < (|j| - 1/2)/K, and
+// 1.41 < 3/2.
 KT_EX double rsqrt_seed(double x) {
 #if defined(__CUDA_ARCH__)
   double y;
@@ -141,9 +151,8 @@ KT_EX double rsqrt_seed(double x) {
 struct Root {
   double g, y;  // RN(sqrt(x)); 1/sqrt(x) within 2^-52
 };
-KT_EX Root make_root(double x) {
+KT_EX Root make_root_seeded(double x, double y0) {
   Root R;
-  const double y0 = rsqrt_seed(x);
   const double e = fma(-(x * y0), y0, 1.0);
   R.y = fma(y0 * e, fma(0.375, e, 0.5), y0);
   const double h = 0.5 * R.y;
@@ -152,11 +161,12 @@ KT_EX Root make_root(double x) {
   R.g = fma(fma(-g, g, x), h, g);
   return R;
 }
-// Bit kTopBit is set when the significand's top 18 bits are all ones or all
-// zeros.
+KT_EX Root make_root(double x) { return make_root_seeded(x, rsqrt_seed(x)); }
+// Bit kTopBit is set when the significand's top 17 bits are all ones or all
+// zeros (x >= 4 (1 - 2^-18) and x < 4 (1 + 2^-17) among them).
 KT_EX uint32_t top_edge(double x) {
   const uint32_t h = hi_word(x);
-  return ((h + 4u) ^ h) | ((h - 4u) ^ h);
+  return ((h + 8u) ^ h) | ((h - 8u) ^ h);
 }
 // 2^-k <= x < 2^k (positive).
 KT_EX bool in_range_pos(double x, int k) {
