@@ -39,6 +39,7 @@ struct Group {
   std::vector<int> frames;  // batch frame indices
   bool fp32 = false;        // some frame may run the mixed FP32 right-hand side
   bool lam = false;         // some frame has Lambda != 0
+  bool tame = true;         // every frame's parameters are Metric::tame
   uint64_t n_rays = 0;
   kt::Frame* d_frames = nullptr;
   kt::OutSoA* d_outs = nullptr;
@@ -104,6 +105,7 @@ kt::BatchRays group_rays(const Group& g, const uint32_t* list, const uint32_t* n
   br.n = n;
   br.fp32 = g.fp32;
   br.lam = g.lam;
+  br.tame = g.tame;
   return br;
 }
 
@@ -323,6 +325,7 @@ kt_status kt_batch_create(kt_context* ctx, const kt_frame_desc* descs, const kt_
     g.frames.push_back(i);
     g.fp32 = g.fp32 || std::isfinite(frames[i].r_fp32);
     g.lam = g.lam || frames[i].g.L != 0.0;
+    g.tame = g.tame && frames[i].g.tame != 0;
     if (frames[i].solver == KT_SOLVER_ELLIPTIC_CLOSED) {
       g.ell_frames.push_back(frames[i]);
       g.ell_outs.push_back(to_out(&outs[i]));

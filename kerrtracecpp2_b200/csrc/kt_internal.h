@@ -148,6 +148,9 @@ struct BatchRays {
   // some frame has Lambda != 0: selects the exact BL kernels that carry
   // Delta_theta and Xi (without it both are 1)
   bool lam = true;
+  // every frame's parameters are within the exact quotients' range
+  // (Metric::tame); otherwise the exact modes' general kernels
+  bool tame = false;
 };
 
 // Launch-shape variants the batch autotuner chooses from: (threads per

@@ -8,10 +8,19 @@
 
 namespace kt {
 
-// The BL modes come in two instantiations: kLam = false for launches whose
+// Instantiations of the exact modes' right-hand sides.  kFlat: launches whose
 // frames all have Lambda = 0 (bl_rhs_exact; 640 x 360 DOPRI5 without Lambda:
-// 14.6 ms, and 14.7 to 15.9 with the Lambda kernel).
-template <class M, bool kLam>
+// 14.6 ms, and 14.7 to 15.9 with the Lambda kernel); kLambda: others.  kGeneral:
+// a frame's parameters lie outside the quotients' range (Metric::tame: |Lambda|
+// below 2^-90, as the observed one is in units of most black holes' masses, a
+// or Q below 2^-40), so that every right-hand side would be evaluated in the
+// exact form, refused and evaluated in the general one by a call (640 x 360
+// DOPRI5 with Lambda = 4.5e-33 26.8 ms, 16.2 with kGeneral; KS with a = 1e-13 at
+// 320 x 180 29.9 and 12.3; 200 x 120 bundles 74 and 45).
+enum Form : int { kFlat = 0, kLambda = 1, kGeneral = 2 };
+static Form form_of(bool lam, bool tame) { return !tame ? kGeneral : lam ? kLambda : kFlat; }
+
+template <class M, Form kForm>
 struct ModeBL {
   using Machine = M;
   static constexpr int kSlots = M::kSlots;
@@ -24,14 +33,18 @@ struct ModeBL {
   __device__ __forceinline__ bool slot(const Frame& f, int s, RayResult* res) {
     double y[4], k[5];
     m->input(s, y);
-    if (!bl_rhs_exact<kLam>(f.g, y[0], y[1], y[2], y[3], m->pt, m->pphi, k))
+    if constexpr (kForm == kGeneral)
+      bl_rhs(f.g, y[0], y[1], y[2], y[3], m->pt, m->pphi, k);
+    else if (!bl_rhs_exact<kForm == kLambda>(f.g, y[0], y[1], y[2], y[3], m->pt, m->pphi, k))
       bl_rhs_rest(f.g, y[0], y[1], y[2], y[3], m->pt, m->pphi, k);
     return m->consume(f, s, k, res);
   }
 };
-template <bool kLam> using ModeBLRk4 = ModeBL<BLRk4, kLam>;
-template <bool kLam> using ModeBLDopri5 = ModeBL<BLDopri5, kLam>;
+template <Form kForm> using ModeBLRk4 = ModeBL<BLRk4, kForm>;
+template <Form kForm> using ModeBLDopri5 = ModeBL<BLDopri5, kForm>;
 
+// (The KS chart has no Lambda: kFlat or kGeneral.)
+template <Form kForm>
 struct ModeKSRk4 {
   using Machine = KSRk4;
   static constexpr int kSlots = KSRk4::kSlots;
@@ -50,7 +63,9 @@ struct ModeKSRk4 {
   __device__ __forceinline__ bool slot(const Frame& f, int s, RayResult* res) {
     double y[6], k[6];
     m->input(s, y);
-    if (!ks_rhs_exact(f.g, y[0], y[1], y[2], y[3], y[4], y[5], m->pT, k))
+    if constexpr (kForm == kGeneral)
+      ks_rhs(f.g, y[0], y[1], y[2], y[3], y[4], y[5], m->pT, k);
+    else if (!ks_rhs_exact(f.g, y[0], y[1], y[2], y[3], y[4], y[5], m->pT, k))
       ks_rhs_rest(f.g, y[0], y[1], y[2], y[3], y[4], y[5], m->pT, k);
     return m->consume(f, s, k, res);
   }
@@ -86,16 +101,22 @@ __device__ __forceinline__ void swap_halves(unsigned mask, const BundleHalf& me,
   for (int i = 0; i < 4; ++i) other->h1[i] = __shfl_xor_sync(mask, me.h1[i], 1);
 }
 
-// The general form, for the states the exact quotients do not take; both
-// lanes of the pair (mask) call it together.
-__device__ __noinline__ void bundle_rhs_pair_rest(const Metric& g, const double y[4], double pt,
-                                                  double pphi, const double W[8], double k[5],
-                                                  double kW[8], bool odd, unsigned mask) {
+// The general form; both lanes of each pair (mask) call it together.
+__device__ __forceinline__ void bundle_rhs_pair_general(const Metric& g, const double y[4], double pt,
+                                                        double pphi, const double W[8], double k[5],
+                                                        double kW[8], bool odd, unsigned mask) {
   BundleHalf me, other;
   bundle_rhs_half(g, y[0], y[1], y[2], y[3], pt, pphi, odd, &me);
   swap_halves(mask, me, &other);
   // the even lane's view (the odd lane's result is not used)
   bundle_rhs_combine(me, other, y[0], y[2], y[3], W, k, kW);
+}
+
+// ... out of line, for the states the exact quotients do not take.
+__device__ __noinline__ void bundle_rhs_pair_rest(const Metric& g, const double y[4], double pt,
+                                                  double pphi, const double W[8], double k[5],
+                                                  double kW[8], bool odd, unsigned mask) {
+  bundle_rhs_pair_general(g, y, pt, pphi, W, k, kW, odd, mask);
 }
 
 template <bool kLam>
@@ -110,7 +131,7 @@ __device__ __forceinline__ void bundle_rhs_paired(const Metric& g, const double 
   if (!__all_sync(pair, ok)) bundle_rhs_pair_rest(g, y, pt, pphi, W, k, kW, odd, pair);
 }
 
-template <bool kLam>
+template <Form kForm>
 struct ModeBundlePair {
   using Machine = Bundle;
   static constexpr int kSlots = Bundle::kSlots;
@@ -124,7 +145,10 @@ struct ModeBundlePair {
                                        unsigned pmask) {
     double y[4], yW[8], k[5], kW[8];
     m->input(s, y, yW);
-    bundle_rhs_paired<kLam>(f.g, y, m->pt, m->pphi, yW, k, kW, odd, pmask);
+    if constexpr (kForm == kGeneral)
+      bundle_rhs_pair_general(f.g, y, m->pt, m->pphi, yW, k, kW, odd, pmask);
+    else
+      bundle_rhs_paired<kForm == kLambda>(f.g, y, m->pt, m->pphi, yW, k, kW, odd, pmask);
     __syncwarp(pmask);  // both lanes have read the record
     int done = 0;
     if (!odd) done = m->consume(f, s, k, kW, res) ? 1 : 0;
@@ -166,7 +190,7 @@ struct ModeSepRk4 {
   }
 };
 
-template <bool kLam> struct Lockstep<ModeBundlePair<kLam>> { static constexpr bool value = true; };
+template <Form kForm> struct Lockstep<ModeBundlePair<kForm>> { static constexpr bool value = true; };
 
 template <> struct Defers<ModeSepRk4> { static constexpr bool value = true; };
 
@@ -184,15 +208,19 @@ template <> struct Defers<ModeSepRk4> { static constexpr bool value = true; };
 // registers without a spill.  720p DOPRI5 41.1 ms against 43.0 with 10 blocks
 // (96 registers, 22 B spilled) and 43.4 with 6; RK4 at 641 x 359 9.4 / 10.7 /
 // 8.8 ms (that frame is short enough for its longest rays to show).
-template <class M, bool kLam> struct Shape<ModeBL<M, kLam>> {
+template <class M, Form kForm> struct Shape<ModeBL<M, kForm>> {
   static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32;
 };
-template <class M, bool kLam> struct BatchMin0<ModeBL<M, kLam>> {
+template <class M, Form kForm> struct BatchMin0<ModeBL<M, kForm>> {
   static constexpr int value = batch_min_blocks(kModeBLRk4, 0);
 };
-template <> struct BatchMin0<ModeKSRk4> { static constexpr int value = batch_min_blocks(kModeKSRk4, 0); };
+template <Form kForm> struct BatchMin0<ModeKSRk4<kForm>> {
+  static constexpr int value = batch_min_blocks(kModeKSRk4, 0);
+};
 // (720p KS frame 51.6 ms against 52.3 with 10 blocks of 96 registers.)
-template <> struct Shape<struct ModeKSRk4> { static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32; };
+template <Form kForm> struct Shape<ModeKSRk4<kForm>> {
+  static constexpr int kBlock = 64, kMinBlocks = 8, kRefill = 32;
+};
 template <> struct Shape<struct ModeBundle> { static constexpr int kBlock = 128, kMinBlocks = 1, kRefill = 16; };
 // Paired bundles: 64 rays per 128-thread block; kRefill counts lanes.
 #ifndef KT_BUNDLE_PAIR_BLOCK
@@ -204,7 +232,7 @@ template <> struct Shape<struct ModeBundle> { static constexpr int kBlock = 128,
 #ifndef KT_BUNDLE_PAIR_REFILL
 #define KT_BUNDLE_PAIR_REFILL 8
 #endif
-template <bool kLam> struct Shape<ModeBundlePair<kLam>> {
+template <Form kForm> struct Shape<ModeBundlePair<kForm>> {
   static constexpr int kBlock = KT_BUNDLE_PAIR_BLOCK, kMinBlocks = KT_BUNDLE_PAIR_MINB,
                        kRefill = KT_BUNDLE_PAIR_REFILL;
 };
@@ -225,13 +253,39 @@ static cudaError_t launch_pair(const Frame& f, const OutSoA& out, const RayList&
   return cudaGetLastError();
 }
 
+// One launch of the mode's instantiation for a form.
+template <template <Form> class ModeF>
+static cudaError_t launch_form(Form form, const Frame& f, const OutSoA& out, const RayList& rl,
+                               uint32_t* queue, const Fallback& fb, const LaunchShape& s,
+                               cudaStream_t stream) {
+  switch (form) {
+    case kFlat: return launch_one<ModeF<kFlat>>(f, out, rl, queue, fb, s, stream);
+    case kLambda: return launch_one<ModeF<kLambda>>(f, out, rl, queue, fb, s, stream);
+    default: return launch_one<ModeF<kGeneral>>(f, out, rl, queue, fb, s, stream);
+  }
+}
+
+template <template <Form> class ModeF>
+static cudaError_t batch_launch_form(Form form, int variant, const BatchRays& br, uint32_t* queue,
+                                     const Fallback& fb, const LaunchShape& s, cudaStream_t st) {
+  switch (form) {
+    case kFlat: return batch_launch<ModeF<kFlat>>(variant, br, queue, fb, s, st);
+    case kLambda: return batch_launch<ModeF<kLambda>>(variant, br, queue, fb, s, st);
+    default: return batch_launch<ModeF<kGeneral>>(variant, br, queue, fb, s, st);
+  }
+}
+
 cudaError_t launch_shape(Mode mode, int device, LaunchShape* shape) {
   if (is_mixed_mode(mode)) return launch_shape_mixed(mode, device, shape);
   switch (mode) {
-    case kModeBLRk4: return shape_for_both<ModeBLRk4<true>, ModeBLRk4<false>>(device, shape);
-    case kModeBLDopri5: return shape_for_both<ModeBLDopri5<true>, ModeBLDopri5<false>>(device, shape);
-    case kModeKSRk4: return shape_for<ModeKSRk4>(device, shape);
-    case kModeBundle: return shape_for_pair<ModeBundlePair<true>, ModeBundlePair<false>>(device, shape);
+    case kModeBLRk4:
+      return shape_for_all<ModeBLRk4<kLambda>, ModeBLRk4<kFlat>, ModeBLRk4<kGeneral>>(device, shape);
+    case kModeBLDopri5:
+      return shape_for_all<ModeBLDopri5<kLambda>, ModeBLDopri5<kFlat>, ModeBLDopri5<kGeneral>>(device, shape);
+    case kModeKSRk4: return shape_for_all<ModeKSRk4<kFlat>, ModeKSRk4<kGeneral>>(device, shape);
+    case kModeBundle:
+      return shape_for_pair<ModeBundlePair<kLambda>, ModeBundlePair<kFlat>, ModeBundlePair<kGeneral>>(device,
+                                                                                                     shape);
     case kModeSepRk4: return shape_for<ModeSepRk4>(device, shape);
     default: return cudaErrorInvalidValue;
   }
@@ -241,25 +295,25 @@ cudaError_t launch_trace(Mode mode, const Frame& f, const OutSoA& out, const Ray
                          uint32_t* queue, const Fallback& fb, const LaunchShape& s,
                          cudaStream_t stream) {
   if (is_mixed_mode(mode)) return launch_trace_mixed(mode, f, out, rl, queue, fb, s, stream);
-  const bool lam = f.g.L != 0.0;
+  const Form form = form_of(f.g.L != 0.0, f.g.tame != 0);
   switch (mode) {
-    case kModeBLRk4:
-      return lam ? launch_one<ModeBLRk4<true>>(f, out, rl, queue, fb, s, stream)
-                 : launch_one<ModeBLRk4<false>>(f, out, rl, queue, fb, s, stream);
-    case kModeBLDopri5:
-      return lam ? launch_one<ModeBLDopri5<true>>(f, out, rl, queue, fb, s, stream)
-                 : launch_one<ModeBLDopri5<false>>(f, out, rl, queue, fb, s, stream);
+    case kModeBLRk4: return launch_form<ModeBLRk4>(form, f, out, rl, queue, fb, s, stream);
+    case kModeBLDopri5: return launch_form<ModeBLDopri5>(form, f, out, rl, queue, fb, s, stream);
     case kModeKSRk4:
+      if (form == kGeneral) return launch_one<ModeKSRk4<kGeneral>>(f, out, rl, queue, fb, s, stream);
       // several lanes per ray where the rays do not fill the device
       // (kt_group.cuh); a count on the device is not known here
       if (!rl.n_dev && rl.n > 0 && rl.n <= kKs8MaxRays)
         return launch_group<GroupKSRk4<8>>(f, out, rl, queue, fb, s.sms, stream);
       if (!rl.n_dev && rl.n > 0 && rl.n <= kKs4MaxRays)
         return launch_group<GroupKSRk4<4>>(f, out, rl, queue, fb, s.sms, stream);
-      return launch_one<ModeKSRk4>(f, out, rl, queue, fb, s, stream);
+      return launch_one<ModeKSRk4<kFlat>>(f, out, rl, queue, fb, s, stream);
     case kModeBundle:
-      return lam ? launch_pair<ModeBundlePair<true>>(f, out, rl, queue, fb, s, stream)
-                 : launch_pair<ModeBundlePair<false>>(f, out, rl, queue, fb, s, stream);
+      switch (form) {
+        case kFlat: return launch_pair<ModeBundlePair<kFlat>>(f, out, rl, queue, fb, s, stream);
+        case kLambda: return launch_pair<ModeBundlePair<kLambda>>(f, out, rl, queue, fb, s, stream);
+        default: return launch_pair<ModeBundlePair<kGeneral>>(f, out, rl, queue, fb, s, stream);
+      }
     case kModeSepRk4: return launch_one<ModeSepRk4>(f, out, rl, queue, fb, s, stream);
     default: return cudaErrorInvalidValue;
   }
@@ -267,15 +321,19 @@ cudaError_t launch_trace(Mode mode, const Frame& f, const OutSoA& out, const Ray
 
 cudaError_t batch_shape(Mode mode, int variant, int device, LaunchShape* shape) {
   switch (mode) {
-    case kModeBLRk4: return batch_shape_both<ModeBLRk4<true>, ModeBLRk4<false>>(variant, device, shape);
+    case kModeBLRk4:
+      return batch_shape_all<ModeBLRk4<kLambda>, ModeBLRk4<kFlat>, ModeBLRk4<kGeneral>>(variant, device,
+                                                                                        shape);
     case kModeBLDopri5:
-      return batch_shape_both<ModeBLDopri5<true>, ModeBLDopri5<false>>(variant, device, shape);
-    case kModeKSRk4: return batch_shape<ModeKSRk4>(variant, device, shape);
+      return batch_shape_all<ModeBLDopri5<kLambda>, ModeBLDopri5<kFlat>, ModeBLDopri5<kGeneral>>(
+          variant, device, shape);
+    case kModeKSRk4:
+      return batch_shape_all<ModeKSRk4<kFlat>, ModeKSRk4<kGeneral>>(variant, device, shape);
     case kModeBundle:
       if (variant == kBatchPairVariant)
-        return batch_shape_pair_for<ModeBundlePair<true>, ModeBundlePair<false>,
-                                    kBatchBlock[kBatchPairVariant],
-                                    kBatchMinBlocks[kBatchPairVariant]>(device, shape);
+        return batch_shape_pair_for<kBatchBlock[kBatchPairVariant], kBatchMinBlocks[kBatchPairVariant],
+                                    ModeBundlePair<kLambda>, ModeBundlePair<kFlat>,
+                                    ModeBundlePair<kGeneral>>(device, shape);
       return batch_shape<ModeBundle>(variant, device, shape);
     case kModeSepRk4: return batch_shape<ModeSepRk4>(variant, device, shape);
     default: return batch_shape_mixed(mode, variant, device, shape);
@@ -284,21 +342,22 @@ cudaError_t batch_shape(Mode mode, int variant, int device, LaunchShape* shape) 
 
 cudaError_t launch_batch(Mode mode, int variant, const BatchRays& br, uint32_t* queue,
                          const Fallback& fb, const LaunchShape& s, cudaStream_t st) {
+  const Form form = form_of(br.lam, br.tame);
   switch (mode) {
-    case kModeBLRk4:
-      return br.lam ? batch_launch<ModeBLRk4<true>>(variant, br, queue, fb, s, st)
-                    : batch_launch<ModeBLRk4<false>>(variant, br, queue, fb, s, st);
-    case kModeBLDopri5:
-      return br.lam ? batch_launch<ModeBLDopri5<true>>(variant, br, queue, fb, s, st)
-                    : batch_launch<ModeBLDopri5<false>>(variant, br, queue, fb, s, st);
-    case kModeKSRk4: return batch_launch<ModeKSRk4>(variant, br, queue, fb, s, st);
+    case kModeBLRk4: return batch_launch_form<ModeBLRk4>(form, variant, br, queue, fb, s, st);
+    case kModeBLDopri5: return batch_launch_form<ModeBLDopri5>(form, variant, br, queue, fb, s, st);
+    case kModeKSRk4:
+      return form == kGeneral ? batch_launch<ModeKSRk4<kGeneral>>(variant, br, queue, fb, s, st)
+                              : batch_launch<ModeKSRk4<kFlat>>(variant, br, queue, fb, s, st);
     case kModeBundle:
       if (variant == kBatchPairVariant) {
         constexpr int kB = kBatchBlock[kBatchPairVariant], kM = kBatchMinBlocks[kBatchPairVariant];
-        if (br.lam)
-          k_trace_batch_pair<ModeBundlePair<true>, kB, kM><<<s.grid, s.block, s.smem, st>>>(br, queue, fb);
+        if (form == kGeneral)
+          k_trace_batch_pair<ModeBundlePair<kGeneral>, kB, kM><<<s.grid, s.block, s.smem, st>>>(br, queue, fb);
+        else if (form == kLambda)
+          k_trace_batch_pair<ModeBundlePair<kLambda>, kB, kM><<<s.grid, s.block, s.smem, st>>>(br, queue, fb);
         else
-          k_trace_batch_pair<ModeBundlePair<false>, kB, kM><<<s.grid, s.block, s.smem, st>>>(br, queue, fb);
+          k_trace_batch_pair<ModeBundlePair<kFlat>, kB, kM><<<s.grid, s.block, s.smem, st>>>(br, queue, fb);
         return cudaGetLastError();
       }
       return batch_launch<ModeBundle>(variant, br, queue, fb, s, st);

@@ -265,25 +265,30 @@ static cudaError_t shape_for(int device, LaunchShape* shape) {
   return cudaSuccess;
 }
 
-// One shape for two instantiations of a mode with the same launch bounds and
-// record (a launch takes either): the larger grid, whose surplus blocks find
-// the queue empty.
-template <class A, class B>
-static cudaError_t shape_for_both(int device, LaunchShape* shape) {
-  LaunchShape b;
-  cudaError_t e = shape_for<A>(device, shape);
-  if (e == cudaSuccess) e = shape_for<B>(device, &b);
-  if (e == cudaSuccess && b.grid > shape->grid) shape->grid = b.grid;
+// One shape for the instantiations of a mode, which share launch bounds and
+// record (a launch takes any of them): the largest grid, whose surplus blocks
+// find the queue empty.
+template <class... Query>
+static cudaError_t largest_grid(LaunchShape* shape, const Query&... query) {
+  cudaError_t e = cudaSuccess;
+  shape->grid = 0;
+  const auto add = [&](const auto& q) {
+    LaunchShape t;
+    if (e == cudaSuccess) e = q(&t);
+    if (e == cudaSuccess && t.grid > shape->grid) *shape = t;
+  };
+  (add(query), ...);
   return e;
 }
 
-template <class A, class B>
+template <class... M>
+static cudaError_t shape_for_all(int device, LaunchShape* shape) {
+  return largest_grid(shape, [=](LaunchShape* t) { return shape_for<M>(device, t); }...);
+}
+
+template <class... M>
 static cudaError_t shape_for_pair(int device, LaunchShape* shape) {
-  LaunchShape b;
-  cudaError_t e = shape_for_pair_one<A>(device, shape);
-  if (e == cudaSuccess) e = shape_for_pair_one<B>(device, &b);
-  if (e == cudaSuccess && b.grid > shape->grid) shape->grid = b.grid;
-  return e;
+  return largest_grid(shape, [=](LaunchShape* t) { return shape_for_pair_one<M>(device, t); }...);
 }
 
 // ---- batches of frames -----------------------------------------------------
@@ -442,13 +447,9 @@ static cudaError_t batch_shape_pair_one(int device, LaunchShape* shape) {
   return cudaSuccess;
 }
 
-template <class A, class B, int BLOCK, int MINB>
+template <int BLOCK, int MINB, class... M>
 static cudaError_t batch_shape_pair_for(int device, LaunchShape* shape) {
-  LaunchShape b;
-  cudaError_t e = batch_shape_pair_one<A, BLOCK, MINB>(device, shape);
-  if (e == cudaSuccess) e = batch_shape_pair_one<B, BLOCK, MINB>(device, &b);
-  if (e == cudaSuccess && b.grid > shape->grid) shape->grid = b.grid;
-  return e;
+  return largest_grid(shape, [=](LaunchShape* t) { return batch_shape_pair_one<M, BLOCK, MINB>(device, t); }...);
 }
 
 template <class ModeT, int BLOCK, int MINB>
@@ -485,14 +486,10 @@ static cudaError_t batch_shape(int variant, int device, LaunchShape* s) {
   return cudaErrorInvalidValue;
 }
 
-// As shape_for_both.
-template <class A, class B>
-static cudaError_t batch_shape_both(int variant, int device, LaunchShape* s) {
-  LaunchShape b;
-  cudaError_t e = batch_shape<A>(variant, device, s);
-  if (e == cudaSuccess) e = batch_shape<B>(variant, device, &b);
-  if (e == cudaSuccess && b.grid > s->grid) s->grid = b.grid;
-  return e;
+// As shape_for_all.
+template <class... M>
+static cudaError_t batch_shape_all(int variant, int device, LaunchShape* s) {
+  return largest_grid(s, [=](LaunchShape* t) { return batch_shape<M>(variant, device, t); }...);
 }
 
 template <class ModeT>
