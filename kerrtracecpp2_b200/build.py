@@ -70,33 +70,33 @@ def build(force=False, verbose=False):
         os.path.join(ROOT, "include", "kerrtrace.h"),
         os.path.join(ROOT, "include", "kerrtrace_cuda_render.h")]
     objs = []
-    jobs = []  # (command, is_nvcc)
+    jobs = []  # (command, file for the compiler's resource listing or None)
     for src in CU_SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src + ".o")
         if force or newer(o, [s] + hdrs):
             flags = [f for f in NVCC_FLAGS if not (src in CU_FLAGS and f == "--fmad=false")]
-            jobs.append(([NVCC] + flags + CU_FLAGS.get(src, []) + ["-c", s, "-o", o], True))
+            jobs.append(([NVCC] + flags + CU_FLAGS.get(src, []) + ["-c", s, "-o", o], o + ".log"))
         objs.append(o)
     for src in CXX_SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src + ".o")
         if force or newer(o, [s] + hdrs):
-            jobs.append((["g++"] + CXX_FLAGS + CXX_FILE_FLAGS.get(src, []) + ["-c", s, "-o", o], False))
+            jobs.append((["g++"] + CXX_FLAGS + CXX_FILE_FLAGS.get(src, []) + ["-c", s, "-o", o], None))
         objs.append(o)
     # Translation units compile independently: run them in parallel.
     with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(len(jobs), os.cpu_count() or 1))) as ex:
         outs = list(ex.map(lambda j: run(j[0], verbose), jobs))
-    ptxas_log = [o for o, (_, is_nvcc) in zip(outs, jobs) if is_nvcc]
+    for out, (_, log) in zip(outs, jobs):
+        if log:
+            with open(log, "w") as f:
+                f.write(out)
     if force or newer(LIB, objs):
         run([NVCC] + ARCH + ["-shared", "-o", LIB] + objs + ["-lgomp"], verbose)
     cli_src = os.path.join(PKG, "cli", "kerr_tracer.cpp")
     if os.path.exists(cli_src) and (force or newer(CLI, [cli_src, LIB] + hdrs)):
         run(["g++", "-O2", "-std=c++17", "-Wall", "-o", CLI, cli_src, "-L", PKG, "-lkerrtrace",
              "-Wl,-rpath,$ORIGIN/.."], verbose)
-    if ptxas_log:
-        with open(os.path.join(BUILD, "ptxas.log"), "w") as f:
-            f.write("\n".join(ptxas_log))
     return LIB
 
 

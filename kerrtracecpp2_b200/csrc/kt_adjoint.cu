@@ -248,8 +248,8 @@ cudaError_t launch_smooth(const Frame& f, const OutSoA& out, uint32_t n, const S
   }
   if (f.chart == 0 && !(job && job->force_bl)) {
     // KS pass over all pixels, then BL over the rays whose KS init failed
-    cudaError_t e = grad ? smooth_launch<ChartKS, true>(f, out, n, jb, jb.pix, jb.n_pix, nullptr, counters,
-                                                        fb_pix, counters + 2, device, st)
+    cudaError_t e = grad ? smooth_launch<ChartKS, true, SmRk4T<true>>(f, out, n, jb, jb.pix, jb.n_pix, nullptr,
+                                                                      counters, fb_pix, counters + 2, device, st)
                          : smooth_launch<ChartKS, false>(f, out, n, jb, jb.pix, jb.n_pix, nullptr, counters,
                                                          fb_pix, counters + 2, device, st);
     if (e != cudaSuccess) return e;

@@ -180,7 +180,7 @@ KT_HD_CALL void sm_paths(double M, const SmPrm<double>& P, const double* c, cons
 
 // One adaptive attempt from (y, pas) with k1 = f(y) and step *h:
 // err = |A - B| / 15, doubling_update; on acceptance (yo, paso) = B.
-template <class C>
+template <class C, bool kPlainPow = false>
 KT_HD int sm_attempt(double M, const SmPrm<double>& P, double tol, const double* c, const double* y,
                      double pas, const double* k1, double k1p, double* h, double* yo, double* paso) {
   double yA[C::kN], yB[C::kN], dAB[C::kN], pB = 0.0;
@@ -190,7 +190,7 @@ KT_HD int sm_attempt(double M, const SmPrm<double>& P, double tol, const double*
     const double d = dAB[i];
     e2 = e2 + d * d;
   }
-  const int res = doubling_update(sqrt(e2) / 15.0, tol, h);
+  const int res = doubling_update<kPlainPow>(sqrt(e2) / 15.0, tol, h);
   if (res == 1) {
     for (int i = 0; i < C::kN; ++i) yo[i] = yB[i];
     *paso = pB;
@@ -318,7 +318,9 @@ KT_HD int sm_attempt_dp(double M, const SmPrm<double>& P, double tol, const doub
   return res;
 }
 
-struct SmRk4;
+template <bool kPlainPow>
+struct SmRk4T;
+typedef SmRk4T<false> SmRk4;
 struct SmDp5;
 
 // Outputs of a stop without event: {ESCAPED, r, 1, theta, phi} of the state.
@@ -855,12 +857,14 @@ KT_HD double sm_attempt_bwd_dp(const Frame& f, const SmPrm<double>& P, const dou
 }
 
 // The integrators of the smooth tracer: an attempt and its reverse.
-struct SmRk4 {
+// kPlainPow: doubling_update's (the KS gradient kernel).
+template <bool kPlainPow>
+struct SmRk4T {
   template <class C>
   KT_HD static int attempt(double M, const SmPrm<double>& P, double tol, const double* c, const double* y,
                            double pas, const double* k1, double k1p, double* h, double* yo,
                            double* paso) {
-    return sm_attempt<C>(M, P, tol, c, y, pas, k1, k1p, h, yo, paso);
+    return sm_attempt<C, kPlainPow>(M, P, tol, c, y, pas, k1, k1p, h, yo, paso);
   }
   template <class C>
   KT_HD static double attempt_bwd(const Frame& f, const SmPrm<double>& P, const double* c,
