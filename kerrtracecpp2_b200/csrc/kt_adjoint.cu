@@ -43,8 +43,22 @@ constexpr int kSumThreads = 256;
 // wait for instructions (their loops are larger than the instruction cache;
 // half the warps per SM are as fast), and a warp that follows another finds
 // them fetched.  640x360 DOPRI5 26.7 -> 23.5 ms, 320x180 bundles 68.9 ->
-// 66.0; groups of 64 or 128 gained nothing.  Fewer rays than 256 per SM leave
-// SMs without a block and keep the 64-thread ones.
+// 66.0; groups of 64 or 128 gained nothing.  But a block waits for its longest
+// ray, and few rays leave a last round of blocks alone on the device: from
+// which count on, in rays per SM (one block of 256 is resident on each), the
+// gradient is faster.  Measured, 64 / 256 threads (ms; two scenes each):
+//   rays       38000        60000        90000        113000       150000       205000
+//   KS       19.0 / 18.4  19.8 / 18.9  20.3 / 19.3  21.0 / 22.3  25.7 / 26.3  30.9 / 31.3
+//            15.1 / 15.0  16.8 / 18.1  17.2 / 17.1  18.0 / 16.9  20.9 / 19.1  22.2 / 22.8
+//   BL RK4   16.3 / 16.0  18.5 / 18.8  20.6 / 22.2  21.5 / 20.8  23.4 / 20.8  25.2 / 20.5
+//            13.6 / 12.5  16.3 / 19.0  15.9 / 16.7  20.2 / 21.0  20.9 / 20.7  26.2 / 25.6
+//   DOPRI5   13.1 / 13.1  15.2 / 15.2  15.0 / 16.1  16.6 / 16.4  17.1 / 15.5  20.4 / 17.5
+//            11.7 / 11.6  11.8 / 12.2  13.7 / 13.7  15.6 / 15.0  18.1 / 16.6  17.8 / 15.6
+// and bundles 66 / 66, 70 / 69 (57600), 69 / 68 (76000), 90 / 91: BL from 1024
+// on, where it is never slower, KS and bundles from 256 on, 2% on the average.
+template <class C>
+constexpr uint32_t kSmWideRays = (C::kN == 6 || C::kBundle) ? 256 : 1024;
+
 template <class C, bool kGrad, class I, int kBlock>
 __global__ void __launch_bounds__(kBlock) k_smooth(const Frame f, const OutSoA out, const SmJob job,
                                                      uint32_t n, const uint32_t* __restrict__ list,
@@ -201,7 +215,7 @@ static cudaError_t smooth_launch(const Frame& f, const OutSoA& out, uint32_t n, 
   int sms = 0;
   const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
-  if (kGrad && !n_dev && (list ? n_list : n) >= (uint32_t)kSmWide * (uint32_t)sms)
+  if (kGrad && !n_dev && (list ? n_list : n) >= kSmWideRays<C> * (uint32_t)sms)
     return smooth_launch_as<C, kGrad, I, kGrad ? kSmWide : kSmBlock>(f, out, n, job, list, n_list, n_dev,
                                                                      queue, fb_pix, fb_n, sms, st);
   return smooth_launch_as<C, kGrad, I, kSmBlock>(f, out, n, job, list, n_list, n_dev, queue, fb_pix, fb_n,
