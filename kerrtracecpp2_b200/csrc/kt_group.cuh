@@ -13,11 +13,19 @@
 // value comes from the expressions of the one-lane machine (KSRk4): the
 // results are the same bit for bit.
 //
-// Measured (ms; one lane with 8 blocks per SM, 4 lanes, 8 lanes):
-//   48 x 27  4.2  2.2  1.9      256 x 144  6.6  4.5  5.3      426 x 240   8.4  10.5  12.9
-//  160 x 90  5.6  3.1  3.1      320 x 180  8.2  6.8  7.7      512 x 512  17.3  24.4  30.7
-// so 8 lanes up to 8192 rays, 4 up to 80000, one above: there the lanes are
-// full anyway and the bookkeeping of a ray is paid by every lane of its group.
+// The rules are by rays per SM, 8 lanes up to 90 and 4 up to 540, one above:
+// there the lanes are full anyway and the bookkeeping of a ray is paid by every
+// lane of its group.  Measured on 148 SMs (ms; 8 lanes / 4 / one with 8 blocks
+// per SM), the frames of three scenes:
+//    4000 rays   2.2 / 2.3 / 5.5    1.9 / 2.1 / 5.6    3.1 / 3.3 / 7.7
+//   12000        2.7 / 2.9 / 6.3    2.4 / 2.7 / 5.7    3.0 / 3.3 / 6.6
+//   16000        3.4 / 3.1 / 6.9    2.9 / 2.9 / 6.0    3.1 / 3.4 / 6.9
+//   24000        4.7 / 4.3 / 8.5    3.6 / 3.5 / 6.9    4.1 / 4.0 / 7.8
+//   57600        7.5 / 7.0 / 9.1    7.8 / 6.8 / 7.3    7.2 / 6.3 / 9.1
+//   72000        9.0 / 7.3 / 8.5    9.5 / 7.8 / 7.6    8.7 / 7.2 / 10.5
+//   80000        9.8 / 8.1 / 8.9   10.5 / 8.6 / 7.8    9.5 / 7.9 / 9.3
+//   90000       11.1 / 9.0 / 8.8   11.7 / 9.5 / 8.1   10.6 / 8.7 / 10.3
+//  100000       12.2 / 9.9 / 10.1  12.9 / 10.5 / 8.9  11.6 / 9.5 / 10.4
 // (A BL form, 4 lanes on the five points, measured no faster at any size: the
 // one-lane right-hand side already has five independent metrics in flight.)
 //
@@ -302,8 +310,7 @@ struct GroupKSRk4 {
 
 // ---- the persistent loop -----------------------------------------------------
 constexpr int kGroupBlock = 64;
-constexpr uint32_t kKs8MaxRays = 8192, kKs4MaxRays = 80000;
-
+constexpr uint32_t kKs8RaysPerSm = 90, kKs4RaysPerSm = 540;
 
 // Blocks per SM: 8 lanes at 128 registers; 4 lanes, which carry two points at a
 // time, at 160 without a spill (320 x 180: 6.8 ms against 7.0 with 8 blocks).

@@ -303,9 +303,9 @@ cudaError_t launch_trace(Mode mode, const Frame& f, const OutSoA& out, const Ray
       if (form == kGeneral) return launch_one<ModeKSRk4<kGeneral>>(f, out, rl, queue, fb, s, stream);
       // several lanes per ray where the rays do not fill the device
       // (kt_group.cuh); a count on the device is not known here
-      if (!rl.n_dev && rl.n > 0 && rl.n <= kKs8MaxRays)
+      if (!rl.n_dev && rl.n > 0 && rl.n <= kKs8RaysPerSm * (uint32_t)s.sms)
         return launch_group<GroupKSRk4<8>>(f, out, rl, queue, fb, s.sms, stream);
-      if (!rl.n_dev && rl.n > 0 && rl.n <= kKs4MaxRays)
+      if (!rl.n_dev && rl.n > 0 && rl.n <= kKs4RaysPerSm * (uint32_t)s.sms)
         return launch_group<GroupKSRk4<4>>(f, out, rl, queue, fb, s.sms, stream);
       return launch_one<ModeKSRk4<kFlat>>(f, out, rl, queue, fb, s, stream);
     case kModeBundle:
