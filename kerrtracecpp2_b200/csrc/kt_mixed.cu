@@ -149,12 +149,17 @@ template <bool B> struct Shape<ModeBLDopri5MixedT<B>> {
   static constexpr int kBlock = 64, kMinBlocks = KT_MIXED_DOPRI5_MINB,
                        kRefill = B ? KT_MIXED32_DOPRI5_REFILL : 32;
 };
-// KS with the FP32 branch, where the rays give every SM a block: 256-thread
-// blocks whose warps go through the slots together (Lockstep; 512 x 512 5.6 ms,
-// 5.8 as 320 x 2, 6.6 as 128 x 5, against 7.0 free-running as 64 x 9).
-// Fewer rays spread over the SMs as free-running blocks of 64 (40 x 30: 2.7 ms
-// against 2.9).  Without the branch 8 blocks of 64 (512 x 512 at tol 1e-9: 3.9 ms
-// against 4.0 with 10).
+// KS with the FP32 branch, from 192 rays per SM on: 256-thread blocks whose
+// warps go through the slots together (Lockstep; 512 x 512 6.8 ms, 6.9 as 320 x
+// 2, 7.8 as 128 x 5, against 8.1 free-running as 64 x 9).  Fewer rays spread
+// over the SMs as free-running blocks of 64.  Measured on 148 SMs (ms of the
+// call, free-running / lockstep, three scenes):
+//   12000 rays  3.1 / 3.1   2.3 / 2.7   3.4 / 3.5     37000  3.8 / 3.7   3.2 / 2.9   4.7 / 4.6
+//   24000       4.2 / 4.2   2.8 / 2.8   4.1 / 4.1     57600  4.6 / 3.9   3.4 / 2.9   4.6 / 4.2
+//   30000       4.1 / 3.8   3.1 / 2.9   3.7 / 3.5    130000  4.9 / 4.3   4.2 / 3.6   5.7 / 5.2
+// Without the branch 8 blocks of 64 (512 x 512 at tol 1e-9: 3.9 ms against 4.0
+// with 10).
+constexpr int kKsLockstepRaysPerSm = 192;
 template <> struct Shape<ModeKSRk4MixedT<true, true>> { static constexpr int kBlock = 256, kMinBlocks = 2, kRefill = 32; };
 template <> struct Lockstep<ModeKSRk4MixedT<true, true>> { static constexpr bool value = true; };
 template <> struct Shape<ModeKSRk4MixedT<true>> { static constexpr int kBlock = 64, kMinBlocks = 9, kRefill = 32; };
@@ -210,7 +215,7 @@ cudaError_t launch_trace_mixed(Mode mode, const Frame& f, const OutSoA& out, con
                   : launch_one<ModeBLDopri5MixedT<false>>(f, out, rl, queue, fb, s, stream);
     case kModeKSRk4Mixed:
       if (!fp32) return launch_one<ModeKSRk4MixedT<false>>(f, out, rl, queue, fb, s, stream);
-      return !rl.n_dev && rl.n < (uint32_t)(256 * s.sms)
+      return !rl.n_dev && rl.n < (uint32_t)(kKsLockstepRaysPerSm * s.sms)
                  ? launch_ks<ModeKSRk4MixedT<true>>(f, out, rl, queue, fb, s, stream)
                  : launch_ks<ModeKSRk4MixedT<true, true>>(f, out, rl, queue, fb, s, stream);
     case kModeBundleMixed: return launch_trace_mixed_bundle(f, out, rl, queue, fb, s, stream);

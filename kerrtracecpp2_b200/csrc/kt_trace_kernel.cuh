@@ -76,7 +76,7 @@ template <class ModeT> struct Shape { static constexpr int kBlock = 128, kMinBlo
 // holds, so that free-running warps, each at its own place in it, fetch it from
 // the next level over and over; side by side they fetch it once.  Measured:
 // two-lane bundles 960 x 540 83.1 -> 76.9 ms (no-instruction stalls 1.1 per
-// issue before), mixed KS 512 x 512 7.0 -> 5.6 ms (7.2 per issue).  The other
+// issue before), mixed KS 512 x 512 8.1 -> 6.8 ms (7.2 per issue).  The other
 // kernels' loops fit, and the barriers cost them (BL DOPRI5 720p 38.0 -> 40.1,
 // KS 51.6 -> 53.9, mixed DOPRI5 14.7 -> 17.3).
 template <class ModeT> struct Lockstep { static constexpr bool value = false; };
