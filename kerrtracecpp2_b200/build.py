@@ -34,7 +34,8 @@ CU_SOURCES = ["kt_kernels.cu", "kt_noalloc.cu", "kt_mixed.cu",
               "kt_mixed_bundle.cu", "kt_adjoint.cu"]
 CXX_SOURCES = ["kt_frame.cpp", "kt_api.cpp", "kt_batch.cpp", "kt_grad.cpp", "kt_io.cpp",
                "kt_compat.cpp"]
-HEADERS = ["ktmath.h", "kt_exact.cuh", "kt_group.cuh", "ktmath_consts.h", "kt_physics.cuh", "kt_machines.cuh", "kt_internal.h",
+HEADERS = ["ktmath.h", "kt_exact.cuh", "kt_group.cuh", "ktmath_consts.h", "kt_physics.cuh",
+           "kt_machines.cuh", "kt_internal.h", "kt_batch_order.h",
            "kt_frame.h", "kt_context.h", "kt_trace_kernel.cuh", "kt_dual.cuh", "kt_smooth.cuh",
            "kt_smray.cuh", "kt_adjoint.h", "kt_elliptic.cuh"]
 # Per-file compile flags: the exact kernels keep every multiply and add of

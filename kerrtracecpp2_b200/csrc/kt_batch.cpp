@@ -362,16 +362,29 @@ kt_status kt_batch_create(kt_context* ctx, const kt_frame_desc* descs, const kt_
   bytes = align256(bytes + counters_bytes);
   const size_t off_scratch = bytes;
   bytes = align256(bytes + ring_scratch * sizeof(uint32_t));
-  // the largest interleaved group's rays, frame after frame (in the batch's one
-  // allocation: an allocation and a free of its own cost the set-up 1 ms)
+  // for the interleaved groups: one group's rays, frame after frame (a group
+  // with a fallback list has them there, which is empty until a launch; in the
+  // batch's one allocation: an allocation and a free of its own cost the set-up
+  // 1 ms), and the tables of the order
   uint64_t n_largest = 0;
-  for (const Group& g : b->groups)
-    if (interleaved(g)) n_largest = std::max(n_largest, g.n_rays);
+  size_t n_words = 0;
+  std::vector<std::vector<uint32_t>> tables(b->groups.size());
+  std::vector<kt::BatchOrder> orders(b->groups.size());
+  for (size_t gi = 0; gi < b->groups.size(); ++gi) {
+    const Group& g = b->groups[gi];
+    if (!interleaved(g)) continue;
+    std::vector<uint64_t> sizes;
+    for (int i : g.frames) sizes.push_back((uint64_t)descs[i].width * (uint64_t)descs[i].height);
+    orders[gi] = kt::make_batch_order(sizes, &tables[gi]);
+    n_words = std::max(n_words, orders[gi].n_words);
+    if (!kt::has_fallback(g.mode)) n_largest = std::max(n_largest, g.n_rays);
+  }
   const size_t off_seq = bytes;
   bytes = align256(bytes + n_largest * sizeof(uint32_t));
+  const size_t off_tables = bytes;
+  bytes = align256(bytes + n_words * sizeof(uint32_t));
   KT_CUDA(ctx, cudaMalloc((void**)&b->d_mem, bytes), "batch buffers");
   uint32_t* d_counters = (uint32_t*)(b->d_mem + off_counters);
-  uint32_t* d_seq = (uint32_t*)(b->d_mem + off_seq);
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
     Group& g = b->groups[gi];
     const size_t nf = g.frames.size();
@@ -396,16 +409,22 @@ kt_status kt_batch_create(kt_context* ctx, const kt_frame_desc* descs, const kt_
             "batch outputs");
     KT_CUDA(ctx, cudaMemcpy(g.d_offsets, hoff.data(), (nf + 1) * sizeof(uint64_t),
                             cudaMemcpyHostToDevice), "batch offsets");
+    uint32_t* d_seq = g.d_order;
+    if (interleaved(g)) d_seq = g.d_fb ? g.d_fb : (uint32_t*)(b->d_mem + off_seq);
     for (size_t k = 0; k < nf; ++k) {
       const kt_frame_desc& dk = descs[g.frames[k]];
       KT_CUDA(ctx, kt::launch_ring_order(dk.width, dk.height, (uint32_t)hoff[k],
                                          (uint32_t*)(b->d_mem + off_scratch),
-                                         (interleaved(g) ? d_seq : g.d_order) + hoff[k],
-                                         ctx->stream), "ray order");
+                                         d_seq + hoff[k], ctx->stream), "ray order");
     }
-    if (interleaved(g))
-      KT_CUDA(ctx, kt::launch_batch_order(g.d_offsets, (int)nf, g.n_rays, d_seq, g.d_order, ctx->stream),
+    if (interleaved(g)) {
+      kt::BatchOrder o = orders[gi];
+      o.words = (const uint32_t*)(b->d_mem + off_tables);
+      KT_CUDA(ctx, cudaMemcpyAsync(b->d_mem + off_tables, tables[gi].data(), o.n_words * sizeof(uint32_t),
+                                   cudaMemcpyHostToDevice, ctx->stream), "ray order");
+      KT_CUDA(ctx, kt::launch_batch_order(o, g.n_rays, g.d_offsets, d_seq, g.d_order, ctx->stream),
               "ray order");
+    }
     KT_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "ray order");
     if (kt::has_fallback(g.mode)) {
       g.fb_variant = default_variant(g.fb_mode);

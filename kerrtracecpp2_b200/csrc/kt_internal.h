@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kt_batch_order.h"
 #include "kt_machines.cuh"
 
 namespace kt {
@@ -193,8 +194,9 @@ cudaError_t launch_batch_mixed_bundle(int variant, const BatchRays& br, uint32_t
 // centre-out order) then start early, where the frames in sequence left the
 // last one's for the end of the launch (12 Kerr frames of 256 x 256 41.6 ms,
 // 37.2 interleaved).  The rays beyond a frame's last whole chunk come at the
-// end.  offsets: the frames' first rays (n_frames + 1).
-cudaError_t launch_batch_order(const uint64_t* offsets, int n_frames, uint64_t n_rays,
+// end.  offsets: the frames' first rays (n_frames + 1); order: tables on the
+// device (kt_batch_order.h).
+cudaError_t launch_batch_order(const BatchOrder& order, uint64_t n_rays, const uint64_t* offsets,
                                const uint32_t* in, uint32_t* out, cudaStream_t stream);
 
 // Centre-out ray order (kt_kernels.cu): base + the W x H frame's pixels in
