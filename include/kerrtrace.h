@@ -289,8 +289,8 @@ kt_status kt_camera_spp_offsets(int32_t camera_spp, double* xy);
  * kernel has -- other groups given variant 3 take their default variant, and
  * the tuner times it for bundle groups only.  With KT_BATCH_AUTOTUNE,
  * kt_batch_create times every variant x threshold on a sample of the group's
- * rays (tune_fraction of them, in runs of 256 neighbouring pixels) and keeps
- * the fastest; the sample's results are written to the outputs.  Otherwise
+ * rays (tune_fraction of them, in chunks of 32 spread over the order of the
+ * launch) and keeps the fastest; the sample's results are written to the outputs.  Otherwise
  * the variant and threshold are the options' (or the single-frame defaults).
  *
  * The graph reads the frames' parameters and output pointers from device

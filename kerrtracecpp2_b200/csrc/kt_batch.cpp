@@ -28,7 +28,7 @@ using namespace ktc;
 
 namespace {
 
-constexpr uint32_t kSampleRun = 256;     // neighbouring rays per tuning run
+constexpr uint32_t kSampleRun = 256;     // a tuning sample's size is a multiple (few rays: all)
 constexpr int kRefillCandidates[] = {1, 16, 24, 32};
 constexpr uint64_t kMaxGroupRays = 1ull << 31;
 static_assert(KT_BATCH_VARIANTS == kt::kBatchVariants, "variant count of the ABI");
@@ -132,17 +132,17 @@ cudaError_t enqueue_group(const Group& g, int variant, const kt::LaunchShape& s,
 }
 
 // Time the candidates (variant x regroup threshold) on a sample of the
-// group's rays and keep the fastest.
+// group's rays and keep the fastest.  The sample is taken from the order that
+// the launch takes them in (centre-out, interleaved), 32 at a time.
 kt_status tune_group(kt_context* ctx, Group& g, const kt_batch_options& opt) {
   const uint64_t n = g.n_rays;
   uint64_t stride_runs = (uint64_t)(1.0 / opt.tune_fraction + 0.5);
   if (stride_runs < 1) stride_runs = 1;
-  std::vector<uint32_t> sample;
-  for (uint64_t run = 0; run * kSampleRun < n; run += stride_runs)
-    for (uint64_t k = run * kSampleRun; k < std::min(n, (run + 1) * kSampleRun); ++k)
-      sample.push_back((uint32_t)k);
+  const uint64_t whole = n / 32, runs = (n + kSampleRun - 1) / kSampleRun;
+  const uint64_t m = std::min(whole, (runs + stride_runs - 1) / stride_runs * (kSampleRun / 32));
+  const uint64_t n_sample = m ? 32 * m : n;  // fewer than 32 rays: all of them
   uint32_t* d_sample = nullptr;
-  KT_CUDA(ctx, cudaMalloc((void**)&d_sample, sample.size() * sizeof(uint32_t)), "tuning sample");
+  KT_CUDA(ctx, cudaMalloc((void**)&d_sample, n_sample * sizeof(uint32_t)), "tuning sample");
   struct Guard {
     uint32_t* p;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -153,8 +153,11 @@ kt_status tune_group(kt_context* ctx, Group& g, const kt_batch_options& opt) {
     }
   } guard{d_sample};
   cudaStream_t st = ctx->stream;
-  KT_CUDA(ctx, cudaMemcpyAsync(d_sample, sample.data(), sample.size() * sizeof(uint32_t),
-                               cudaMemcpyHostToDevice, st), "tuning sample");
+  if (m)
+    KT_CUDA(ctx, kt::launch_sample_order(g.d_order, whole, m, d_sample, st), "tuning sample");
+  else
+    KT_CUDA(ctx, cudaMemcpyAsync(d_sample, g.d_order, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st),
+            "tuning sample");
   KT_CUDA(ctx, cudaEventCreate(&guard.e0), "event");
   KT_CUDA(ctx, cudaEventCreate(&guard.e1), "event");
   kt::LaunchShape shapes[kt::kBatchVariants];
@@ -163,7 +166,7 @@ kt_status tune_group(kt_context* ctx, Group& g, const kt_batch_options& opt) {
     KT_CUDA(ctx, kt::batch_shape(g.mode, v, ctx->device, &shapes[v]), "occupancy query");
     // Untimed first launch of each variant (module load, caches).
     KT_CUDA(ctx, cudaMemsetAsync(g.d_counters, 0, 4 * sizeof(uint32_t), st), "reset queue");
-    KT_CUDA(ctx, enqueue_group(g, v, shapes[v], 1, d_sample, std::min<uint64_t>(sample.size(), 4096),
+    KT_CUDA(ctx, enqueue_group(g, v, shapes[v], 1, d_sample, std::min<uint64_t>(n_sample, 4096),
                                st), "tuning launch");
   }
   const int reps = std::max(1, opt.tune_reps);
@@ -176,7 +179,7 @@ kt_status tune_group(kt_context* ctx, Group& g, const kt_batch_options& opt) {
       for (int r = 0; r < reps; ++r) {
         KT_CUDA(ctx, cudaMemsetAsync(g.d_counters, 0, 4 * sizeof(uint32_t), st), "reset queue");
         KT_CUDA(ctx, cudaEventRecord(guard.e0, st), "event");
-        KT_CUDA(ctx, enqueue_group(g, v, shapes[v], rm, d_sample, sample.size(), st),
+        KT_CUDA(ctx, enqueue_group(g, v, shapes[v], rm, d_sample, n_sample, st),
                 "tuning launch");
         KT_CUDA(ctx, cudaEventRecord(guard.e1, st), "event");
         KT_CUDA(ctx, cudaEventSynchronize(guard.e1), "tuning run");
@@ -196,7 +199,7 @@ kt_status tune_group(kt_context* ctx, Group& g, const kt_batch_options& opt) {
   g.shape = shapes[g.variant];
   g.info.tuned = 1;
   g.info.candidates = candidates;
-  g.info.sample_rays = (double)sample.size();
+  g.info.sample_rays = (double)n_sample;
   g.info.best_ms = best;
   g.info.default_ms = dflt;
   return KT_OK;

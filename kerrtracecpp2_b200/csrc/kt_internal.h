@@ -199,6 +199,10 @@ cudaError_t launch_batch_mixed_bundle(int variant, const BatchRays& br, uint32_t
 cudaError_t launch_batch_order(const BatchOrder& order, uint64_t n_rays, const uint64_t* offsets,
                                const uint32_t* in, uint32_t* out, cudaStream_t stream);
 
+// m of the `whole` chunks of 32 rays of an order list, spread over it.
+cudaError_t launch_sample_order(const uint32_t* order, uint64_t whole, uint64_t m, uint32_t* sample,
+                                cudaStream_t stream);
+
 // Centre-out ray order (kt_kernels.cu): base + the W x H frame's pixels in
 // rings about the image centre, innermost first, in blocks of 8 x 4 pixels
 // within a ring, into `list` (W*H words); `scratch` holds

@@ -566,6 +566,28 @@ cudaError_t launch_batch_order(const BatchOrder& order, uint64_t n_rays, const u
   return cudaGetLastError();
 }
 
+// Chunks of 32 spread over an order list, one warp each: chunk i of m lies at
+// (i + f) whole / m, f the fractional part of i times the golden ratio (a fixed
+// stride would meet the same frame of an interleaved list every time).
+__global__ void k_sample_order(const uint32_t* __restrict__ order, uint64_t whole, uint64_t m,
+                               uint32_t* __restrict__ sample) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= m) return;
+  uint64_t at = i;
+  if (m < whole) {
+    const double f = (double)i * 0.6180339887498949;
+    at = min(whole - 1, (uint64_t)(((double)i + (f - floor(f))) * ((double)whole / (double)m)));
+  }
+  sample[i * 32 + lane] = order[at * 32 + lane];
+}
+
+cudaError_t launch_sample_order(const uint32_t* order, uint64_t whole, uint64_t m, uint32_t* sample,
+                                cudaStream_t stream) {
+  k_sample_order<<<(unsigned)((m + 7) / 8), 256, 0, stream>>>(order, whole, m, sample);
+  return cudaGetLastError();
+}
+
 // ---- colour ------------------------------------------------------------------
 
 // One pixel of colorize_buffer (main.cpp:1817-1866), both palettes.  The
