@@ -70,11 +70,10 @@ WORKLOADS = {
 # camera azimuths, traced as one batch.
 BATCH_720P_FRAMES = 8
 
-# Algorithmic FP64 work, counted from the reference's arithmetic as
-# kt_physics.cuh evaluates it (+, -, * = 1 flop, fma = 2), each division,
-# square root, sincos and pow weighted by its cost measured on the device in
-# the same run (kt_measure_op_costs: the FMA-pipe time of one operation at
-# full throughput, in flops):
+# Algorithmic FP64 work of the reference's arithmetic (+, -, * = 1 flop, fma =
+# 2), each division, square root, sincos and pow weighted by its cost measured
+# on the device in the same run (kt_measure_op_costs: the FMA-pipe time of one
+# operation at full throughput, in flops):
 #   BL RHS (geodesic_rhs + dphi_vel): 211 flops of arithmetic (5 g^{mu nu}
 #   evaluations: 28 flops full, 21 at the centre, 19 when only theta changes;
 #   4 Hamiltonians of 16; 18 in the three angle factors; 14 for the offsets,
@@ -87,10 +86,28 @@ BATCH_720P_FRAMES = 8
 #   accepted step.
 # With unit weights (division, x/3 and sqrt 1 flop; sincos 70 and pow 113,
 # the flops of their own arithmetic) the counts give 453, 447 and 335.
+# The kernels do less than the weighted counts charge (their quotients share
+# reciprocals): EXEC_* below is what they execute.
 RHS_COUNTS = {"flops": 211.0, "div": 26.0, "div3": 6.0, "sincos": 3.0}
 DOPRI5_ATTEMPT_COUNTS = {"flops": 328.0, "div": 5.0, "sqrt": 1.0, "pow": 1.0}
 RK4_ATTEMPT_COUNTS = {"flops": 219.0, "div": 2.0, "sqrt": 1.0, "pow": 1.0}
 UNIT_WEIGHTS = {"div": 1.0, "div3": 1.0, "sqrt": 1.0, "sincos": 70.0, "pow": 113.0}
+# What bl_rhs_exact (kt_physics.cuh) executes, fma = 2 flops, with and without
+# Lambda: 3 radii (r^2, r^2 + a^2, Delta_r and its product with a^2: 16 / 7),
+# 3 angles (14 / 4, and ktm_sincos_core's 72), 5 inverse metrics (13 / 9 flops
+# of denominators and numerators, 3 reciprocals of 8, 5 quotients of 9 -- 4 and
+# one of 4 without Lambda), 4 Hamiltonians of 14, 36 for the offsets, the two
+# differences' quotients and k.  557 of the 808 flops' operations are FP64
+# instructions; with the attempts' share that makes 16.1 G warp instructions
+# for the 720p headline frame, and ncu counts 16.65 G.
+EXEC_RHS = {True: 3 * 16 + 3 * (14 + 72) + 5 * (13 + 3 * 8 + 5 * 9) + 4 * 14 + 36,
+            False: 3 * 7 + 3 * (4 + 72) + 5 * (9 + 3 * 8 + 4 * 9 + 4) + 4 * 14 + 36}
+# Attempts as executed: DOPRI5's stage sums and results skip zero weights and
+# form y5 once (26 terms of 9 flops), error norm and controller as above; RK4
+# doubling takes three h/6 as ktm_div3 and a halving (6 flops).  Their
+# divisions, root and pow are the device's and ktmath's, at measured cost.
+EXEC_DOPRI5_ATTEMPT = dict(DOPRI5_ATTEMPT_COUNTS, flops=26 * 9.0 + 21 + 1)
+EXEC_RK4_ATTEMPT = dict(RK4_ATTEMPT_COUNTS, flops=219.0 + 3 * 6)
 # DRAM bytes read + written by one k_trace<ModeBL<BLDopri5, true>> launch on
 # the default 720p frame, from one ncu capture of that launch
 # (dram__bytes_read.sum 3.887 MB + dram__bytes_write.sum 8.648 MB): most of
@@ -164,6 +181,48 @@ def ray_flops(desc, steps, attempts, w=UNIT_WEIGHTS):
         return rhs * f_rhs + attempts * weighted(DOPRI5_ATTEMPT_COUNTS, w)
     rhs = n + 10.0 * attempts + steps
     return rhs * f_rhs + attempts * weighted(RK4_ATTEMPT_COUNTS, w)
+
+
+def executed_flops(desc, steps, attempts, w):
+    """FP64 flops that the kernels execute for one traced frame (EXEC_*), with
+    measured weights w for the attempts' divisions, root and pow."""
+    if ray_flops(desc, steps, attempts) is None:
+        return None
+    n = desc.width * desc.height
+    f_rhs = float(EXEC_RHS[desc.Lambda != 0.0])
+    if desc.integrator == 1:
+        return (n + 6.0 * attempts) * f_rhs + attempts * weighted(EXEC_DOPRI5_ATTEMPT, w)
+    return (n + 10.0 * attempts + steps) * f_rhs + attempts * weighted(EXEC_RK4_ATTEMPT, w)
+
+
+def roofline_of(desc, steps, attempts, costs, peak_gflops, kernel_ms):
+    """The roofline of a frame's trace: executed FP64 flops over the kernel's
+    time against the measured FMA peak (None where they are not counted).
+    Beside it the reference's arithmetic with each operation at its measured
+    stand-alone cost (frac_division_equivalent: work the kernels avoid counts
+    as done) and with unit weights."""
+    weights = {k: costs[k] for k in UNIT_WEIGHTS}
+    flops = executed_flops(desc, steps, attempts, weights)
+    if flops is None:
+        return None
+    n = desc.width * desc.height
+    equivalent, unit = ray_flops(desc, steps, attempts, weights), ray_flops(desc, steps, attempts)
+    peak, rate = peak_gflops / 1e3, 1e-12 / (kernel_ms * 1e-3)
+    return {"bound": "fp64", "achieved": flops * rate, "peak": peak, "unit": "TFLOP/s",
+            "frac": flops * rate / peak,
+            "traffic": None,
+            "peak_source": "measured in this run: kt_measure_fp64_peak (dependent FMA chains, all SMs)",
+            "flops_per_frame": flops,
+            "flops_source": "executed by the kernel (fma 2, + - * 1): shared reciprocals, no divisions",
+            "op_weights_flops": {k: round(v, 2) for k, v in weights.items()},
+            "op_weights_source": "measured in this run: kt_measure_op_costs (throughput against FMA)",
+            "frac_division_equivalent": equivalent * rate / peak,
+            "flops_per_frame_division_equivalent": equivalent,
+            "frac_unit_weights": unit * rate / peak,
+            "flops_per_frame_unit_weights": unit,
+            "rhs_per_ray": (n + 6.0 * attempts) / n
+            if desc.integrator == 1 else (n + 10.0 * attempts + steps) / n,
+            "kernel_ms": kernel_ms}
 
 
 ORDER_MIN_PIXELS = 1 << 16  # kt_internal.h kOrderMinPixels
@@ -1034,26 +1093,9 @@ def main():
     steps_sum = float(out["steps"].to(torch.int64).sum())
     att_sum = float(out["attempts"].to(torch.int64).sum())
     costs = R.op_costs()
-    weights = {k: costs[k] for k in UNIT_WEIGHTS}
-    flops = ray_flops(desc, steps_sum, att_sum, weights)
-    flops_unit = ray_flops(desc, steps_sum, att_sum)
-    peak_gflops = R.fp64_peak_gflops()
-    roofline = None
-    if flops is not None:
-        achieved = flops / (kernel_ms * 1e-3) / 1e12
-        peak = peak_gflops / 1e3
-        roofline = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                    "frac": achieved / peak,
-                    "traffic": TRAFFIC_DOPRI5_720P if args.workload == "knds_bl_dopri5_720p" else None,
-                    "peak_source": "measured in this run: kt_measure_fp64_peak (dependent FMA chains, all SMs)",
-                    "flops_per_frame": flops,
-                    "op_weights_flops": {k: round(v, 2) for k, v in weights.items()},
-                    "op_weights_source": "measured in this run: kt_measure_op_costs (throughput against FMA)",
-                    "frac_unit_weights": flops_unit / (kernel_ms * 1e-3) / 1e12 / peak,
-                    "flops_per_frame_unit_weights": flops_unit,
-                    "rhs_per_ray": (n + 6.0 * att_sum) / n
-                    if desc.integrator == 1 else (n + 10.0 * att_sum + steps_sum) / n,
-                    "kernel_ms": kernel_ms}
+    roofline = roofline_of(desc, steps_sum, att_sum, costs, R.fp64_peak_gflops(), kernel_ms)
+    if roofline is not None and args.workload == "knds_bl_dopri5_720p":
+        roofline["traffic"] = TRAFFIC_DOPRI5_720P
 
     # end to end through the public host-buffer call (kt_trace_host): the
     # frame parameters go in, the per-pixel results come back to pinned host
