@@ -37,9 +37,7 @@ def _run(cmd):
 
 def build_all(force=False):
     os.makedirs(BUILD, exist_ok=True)
-    heads = [os.path.join(CSRC, h) for h in ("ktmath.h", "ktmath_consts.h", "kt_physics.cuh",
-                                             "kt_machines.cuh", "kt_frame.h", "kt_dual.cuh",
-                                             "kt_smooth.cuh", "kt_smray.cuh")]
+    heads = [os.path.join(CSRC, h) for h in sorted(os.listdir(CSRC)) if h.endswith((".h", ".cuh"))]
     heads.append(os.path.join(ROOT, "include", "kerrtrace.h"))
     src = os.path.join(TESTS, "ktmath_shim.c")
     if force or _newer(SHIM, [src] + heads):
