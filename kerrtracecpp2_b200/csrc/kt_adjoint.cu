@@ -44,20 +44,28 @@ constexpr int kSumThreads = 256;
 // half the warps per SM are as fast), and a warp that follows another finds
 // them fetched.  640x360 DOPRI5 26.7 -> 23.5 ms, 320x180 bundles 68.9 ->
 // 66.0; groups of 64 or 128 gained nothing.  But a block waits for its longest
-// ray, and few rays leave a last round of blocks alone on the device: from
-// which count on, in rays per SM (one block of 256 is resident on each), the
-// gradient is faster.  Measured, 64 / 256 threads (ms; two scenes each):
-//   rays       38000        60000        90000        113000       150000       205000
-//   KS       19.0 / 18.4  19.8 / 18.9  20.3 / 19.3  21.0 / 22.3  25.7 / 26.3  30.9 / 31.3
-//            15.1 / 15.0  16.8 / 18.1  17.2 / 17.1  18.0 / 16.9  20.9 / 19.1  22.2 / 22.8
-//   BL RK4   16.3 / 16.0  18.5 / 18.8  20.6 / 22.2  21.5 / 20.8  23.4 / 20.8  25.2 / 20.5
-//            13.6 / 12.5  16.3 / 19.0  15.9 / 16.7  20.2 / 21.0  20.9 / 20.7  26.2 / 25.6
-//   DOPRI5   13.1 / 13.1  15.2 / 15.2  15.0 / 16.1  16.6 / 16.4  17.1 / 15.5  20.4 / 17.5
-//            11.7 / 11.6  11.8 / 12.2  13.7 / 13.7  15.6 / 15.0  18.1 / 16.6  17.8 / 15.6
-// and bundles 66 / 66, 70 / 69 (57600), 69 / 68 (76000), 90 / 91: BL from 1024
-// on, where it is never slower, KS and bundles from 256 on, 2% on the average.
+// ray, and few rays leave a last round of blocks alone on the device.  Measured
+// on 148 SMs (one block of 256 is resident on each), 64 / 256 threads (ms; two
+// scenes each):
+//   rays     KS                        BL RK4                    DOPRI5
+//    38000   19.0 / 18.4  15.1 / 15.0  16.3 / 16.0  13.6 / 12.5  13.1 / 13.1  11.7 / 11.6
+//    60000   19.8 / 18.9  16.8 / 18.1  18.5 / 18.8  16.3 / 19.0  15.2 / 15.2  11.8 / 12.2
+//    90000   20.3 / 19.3  17.2 / 17.1  20.6 / 22.2  15.9 / 16.7  15.0 / 16.1  13.7 / 13.7
+//   113000   21.0 / 22.3  18.0 / 16.9  21.5 / 20.8  20.2 / 21.0  16.6 / 16.4  15.6 / 15.0
+//   150000   25.7 / 26.3  20.9 / 19.1  23.4 / 20.8  20.9 / 20.7  17.1 / 15.5  18.1 / 16.6
+//   205000   30.8 / 31.0  22.2 / 22.6  24.1 / 20.2  24.8 / 25.0  25.0 / 22.0  18.0 / 15.2
+//   300000   39.1 / 39.2  27.1 / 27.3  30.3 / 24.9  31.0 / 31.8  31.8 / 26.2  20.7 / 17.7
+//   400000   50.2 / 49.7  32.7 / 32.6  30.6 / 31.5  40.1 / 41.3  30.5 / 32.7  22.5 / 18.3
+//   520000   63.5 / 62.5  39.1 / 40.0  36.7 / 39.1  50.8 / 52.3  37.0 / 41.2  23.0 / 22.4
+//   921600  104.0 / 101.9 64.1 / 65.4  59.3 / 62.5  80.6 / 83.9  61.1 / 67.0  36.5 / 37.0
+// and bundles 66 / 66, 69 / 68 (76000), 139 / 136 (200000), 309 / 304 (518400).
+// So KS and bundles from 256 rays per SM on (1 to 2% on the average), BL between
+// 1024 and 2048 (the 64-thread kernels' own time hardly grows from 205000 to
+// 400000 rays; beyond, side by side costs more than it saves).
 template <class C>
-constexpr uint32_t kSmWideRays = (C::kN == 6 || C::kBundle) ? 256 : 1024;
+constexpr bool sm_wide(uint32_t rays, uint32_t sms) {
+  return (C::kN == 6 || C::kBundle) ? rays >= 256 * sms : rays >= 1024 * sms && rays <= 2048 * sms;
+}
 
 template <class C, bool kGrad, class I, int kBlock>
 __global__ void __launch_bounds__(kBlock) k_smooth(const Frame f, const OutSoA out, const SmJob job,
@@ -215,7 +223,7 @@ static cudaError_t smooth_launch(const Frame& f, const OutSoA& out, uint32_t n, 
   int sms = 0;
   const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
-  if (kGrad && !n_dev && (list ? n_list : n) >= kSmWideRays<C> * (uint32_t)sms)
+  if (kGrad && !n_dev && sm_wide<C>(list ? n_list : n, (uint32_t)sms))
     return smooth_launch_as<C, kGrad, I, kGrad ? kSmWide : kSmBlock>(f, out, n, job, list, n_list, n_dev,
                                                                      queue, fb_pix, fb_n, sms, st);
   return smooth_launch_as<C, kGrad, I, kSmBlock>(f, out, n, job, list, n_list, n_dev, queue, fb_pix, fb_n,

@@ -1,5 +1,5 @@
-"""The line above which gradient rays go 256 to a block: the same rays on both
-sides of it, and single rays' contributions (a cotangent of one pixel), bit for
+"""The lines between which gradient rays go 256 to a block: the same rays on both
+sides of them, and single rays' contributions (a cotangent of one pixel), bit for
 bit."""
 import numpy as np
 import pytest
@@ -12,6 +12,7 @@ KINDS = {
     "ks": (256, dict(chart=0, a=0.7, r_obs=20.0)),
     "rk4": (1024, dict(chart=1, a=0.7, Lambda=1e-4, r_obs=20.0)),
     "dopri5": (1024, dict(chart=1, integrator=1, a=0.7, r_obs=20.0, tol=1e-8)),
+    "rk4_upper": (2048, dict(chart=1, a=0.7, Lambda=1e-4, r_obs=20.0)),
     "bundle": (256, dict(chart=1, bundles=1, a=0.95, theta_deg=60.0, r_obs=20.0, max_steps=400)),
 }
 
