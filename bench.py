@@ -98,8 +98,8 @@ UNIT_WEIGHTS = {"div": 1.0, "div3": 1.0, "sqrt": 1.0, "sincos": 70.0, "pow": 113
 # of denominators and numerators, 3 reciprocals of 8, 5 quotients of 9 -- 4 and
 # one of 4 without Lambda), 4 Hamiltonians of 14, 36 for the offsets, the two
 # differences' quotients and k.  557 of the 808 flops' operations are FP64
-# instructions; with the attempts' share that makes 16.1 G warp instructions
-# for the 720p headline frame, and ncu counts 16.65 G.
+# instructions; with the attempts' share that makes 16.3 G warp instructions
+# for the 720p headline frame, and ncu counts 16.2 G.
 EXEC_RHS = {True: 3 * 16 + 3 * (14 + 72) + 5 * (13 + 3 * 8 + 5 * 9) + 4 * 14 + 36,
             False: 3 * 7 + 3 * (4 + 72) + 5 * (9 + 3 * 8 + 4 * 9 + 4) + 4 * 14 + 36}
 # Attempts as executed: DOPRI5's stage sums and results skip zero weights and

@@ -529,7 +529,7 @@ kt_status kt_render_spp_host(kt_context* ctx, const kt_frame_desc* desc, const k
   br.fp32 = std::isfinite(f.r_fp32);
   br.lam = f.g.L != 0.0;
   br.tame = f.g.tame != 0;
-  // the single-frame launch shapes: 64 x 9 for the exact BL kernels, 128 x 1 otherwise
+  // variant 0 (its blocks per SM: batch_min_blocks) for the BL kernels, 128 x 1 otherwise
   auto variant = [](kt::Mode md) { return (md == kt::kModeBLRk4 || md == kt::kModeBLDopri5) ? 0 : 1; };
   kt::LaunchShape ls;
   KT_CUDA(ctx, kt::batch_shape(m, variant(m), ctx->device, &ls), "occupancy query");

@@ -62,7 +62,8 @@ struct Group {
 int default_variant(kt::Mode m) {
   // The single-frame launch shapes (kt_kernels.cu, kt_mixed.cu): two lanes
   // per ray, 128 x 3, for the FP64 bundle kernel; 128 x 1 for the mixed
-  // bundle and separable-Kerr kernels; 64 x 9 for the others.
+  // bundle and separable-Kerr kernels; for the others 64 threads by
+  // batch_min_blocks (kt_internal.h).
   if (m == kt::kModeBundle) return kt::kBatchPairVariant;
   return (m == kt::kModeBundleMixed || m == kt::kModeSepRk4) ? 1 : 0;
 }

@@ -11,10 +11,12 @@
 // (persistent kernel).  Ray machines live in shared memory; results go out
 // as SoA.
 //
-// The kernels do no waiting on other threads: the only inter-thread
-// operation is the warp-synchronous refill and the queue atomic.  Every ray
-// stops after at most max_steps accepted steps with at most 65 rejected
-// attempts each (the reference's limits), so every loop ends.
+// No kernel waits for another block: the inter-thread operations are the
+// warp-synchronous refill, the queue atomic and, in the modes that go through
+// the slots block by block (Lockstep), barriers of one block whose loop all its
+// threads leave together.  Every ray stops after at most max_steps accepted
+// steps with at most 65 rejected attempts each (the reference's limits), so
+// every loop ends.
 #pragma once
 
 #include "kt_internal.h"
