@@ -26,7 +26,7 @@
 // q0 = RN(a y2), which can be 1.5 ulp off, the bound fails for b_m > 1.15.)
 // The excluded significands (the top 18 bits all ones) are part of the
 // range test; their quotients take the division.  Nothing over- or
-// underflows for |b| in [2^-300, 2^300] and non-zero |a| in [2^-500, 2^500]
+// underflows for |b| in [2^-350, 2^300] and non-zero |a| in [2^-500, 2^500]
 // (the smallest intermediate, a residual, is 2^-106 |a|).
 #pragma once
 

@@ -369,7 +369,7 @@ KT_HD Inv bl_inv_exact(const Metric& g, const BLRad& R, const BLAng& A, uint32_t
   ntp = kLam ? g.axi2 * ntp : g.a * ntp;
   npp = kLam ? g.xi2 * npp : npp;
   *top |= top_ones(sig) | top_ones(pre) | top_ones(p3);
-  *ok = *ok & in_range(pre, 300);
+  *ok = *ok & in_range(pre, 300);  // and so p3 > 2^-347, where it is used (sin^2 > 1e-14)
   const Rcp Rs = make_rcp(sig), Rp = make_rcp(pre), R3 = make_rcp(p3);
   Inv U;
   U.tt = quot(ntt, Rp);

@@ -21,7 +21,7 @@ static __device__ bool differ(const double* a, const double* b) {
 
 // Largest |1 - b y0| (root: |1 - x y0^2| / 2) over every top 20 significand
 // bits, both ends of the range of the low word and every exponent in
-// [-300, 300): for one seed the error is monotone in b, so the ends bound all
+// [-350, 300): for one seed the error is monotone in b, so the ends bound all
 // of it, given that the seed depends on the high word alone (*other: low words
 // with another seed).
 __global__ void k_seeds(bool root, unsigned long long* worst, unsigned long long* other) {
@@ -29,7 +29,7 @@ __global__ void k_seeds(bool root, unsigned long long* worst, unsigned long long
   if (top >= (1u << 20)) return;
   double w = 0.0;
   unsigned long long diff = 0;
-  for (int e = -300; e < 300; ++e) {
+  for (int e = -350; e < 300; ++e) {
     const uint64_t hi = ((uint64_t)(1023 + e) << 52) | ((uint64_t)top << 32);
     const double b0 = ktm_from_bits(hi), b1 = ktm_from_bits(hi | 0xffffffffu);
     const double bm = ktm_from_bits(hi | ((top * 2654435761u) ^ (uint32_t)(e * 40503)));
