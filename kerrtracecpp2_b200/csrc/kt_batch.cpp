@@ -407,12 +407,15 @@ kt_status kt_batch_create(kt_context* ctx, const kt_frame_desc* descs, const kt_
       ho[k] = to_out(&outs[i]);
       hoff[k + 1] = hoff[k] + (uint64_t)descs[i].width * (uint64_t)descs[i].height;
     }
-    KT_CUDA(ctx, cudaMemcpy(g.d_frames, hf.data(), nf * sizeof(kt::Frame), cudaMemcpyHostToDevice),
-            "batch frames");
-    KT_CUDA(ctx, cudaMemcpy(g.d_outs, ho.data(), nf * sizeof(kt::OutSoA), cudaMemcpyHostToDevice),
-            "batch outputs");
-    KT_CUDA(ctx, cudaMemcpy(g.d_offsets, hoff.data(), (nf + 1) * sizeof(uint64_t),
-                            cudaMemcpyHostToDevice), "batch offsets");
+    // on the context's stream, which the order and tuning kernels below run on:
+    // it is a non-blocking one, and a copy on the default stream may still be
+    // on its way from its staging buffer when the call returns
+    KT_CUDA(ctx, cudaMemcpyAsync(g.d_frames, hf.data(), nf * sizeof(kt::Frame), cudaMemcpyHostToDevice,
+                                 ctx->stream), "batch frames");
+    KT_CUDA(ctx, cudaMemcpyAsync(g.d_outs, ho.data(), nf * sizeof(kt::OutSoA), cudaMemcpyHostToDevice,
+                                 ctx->stream), "batch outputs");
+    KT_CUDA(ctx, cudaMemcpyAsync(g.d_offsets, hoff.data(), (nf + 1) * sizeof(uint64_t),
+                                 cudaMemcpyHostToDevice, ctx->stream), "batch offsets");
     uint32_t* d_seq = g.d_order;
     if (interleaved(g)) d_seq = g.d_fb ? g.d_fb : (uint32_t*)(b->d_mem + off_seq);
     for (size_t k = 0; k < nf; ++k) {
